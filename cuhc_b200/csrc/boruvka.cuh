@@ -3,10 +3,15 @@
 // Round structure (the reference runs steps 2-5 on the CPU with two
 // synchronous copies per round, mst.cuh:118-181; here nothing leaves the
 // device but two counters):
-//   1. BVH purity of the current components; each component's best known
-//      edge weight is seeded from last round's per-point edges that now
-//      leave it (a valid upper bound that lets the pass prune at once);
-//   2. the pass: per point, its minimum edge to another component;
+//   1. BVH purity of the current components; every row gets the lightest edge
+//      to another component it already knows (from its k-NN list, or last
+//      round's answer) and a lower bound of every edge it does not know; the
+//      components' best known weights are seeded from those edges;
+//   2. rows that can still matter search: not the settled ones (their known
+//      edge is provably their lightest), not those whose bound exceeds their
+//      component's best, not those of components that sit the round out (see
+//      Participation). The rows left are packed into row tiles of their own,
+//      and the pass finds, per row, its minimum edge to another component;
 //   3. per component, the minimum edge under the order (weight, u, v) with
 //      ORIGINAL indices: an atomicMin over (weight bits << 32 | u), then an
 //      atomicMin over v among the points that hold that (weight, u). Any
@@ -22,8 +27,8 @@
 
 #include <algorithm>
 #include <typeinfo>
-#include <tuple>
 #include <mutex>
+#include <tuple>
 #include <map>
 #include <random>
 #include <type_traits>
@@ -63,92 +68,189 @@ namespace boruvka_detail {
 
 inline int blocks(long long work, int threads = 256) { return (int)((work + threads - 1) / threads); }
 
-static __global__ void iotaKernel(int *a, int n) {
+// Which components search in a round. Borůvka's cut argument holds for every
+// component on its own, so a component may sit a round out: the edges that the
+// others choose are in the tree whatever it does, and whoever joins it spares
+// its rows their search. The largest component of an instance sits out (its
+// edges are found from the other side, by fewer rows), and so does every
+// component of more than twice the instance's mean size: at most half of the
+// components can be that large, so at least half choose an edge and the rounds
+// stay logarithmic. Components under kSitOutMin rows (8 row tiles) always
+// search; their rows cost less than a round. A component that is alone in its
+// instance is done. Arrays are indexed by the instance's root node.
+constexpr int kSitOutMin = 1024;
+
+struct Participation {
+  const int *size = nullptr;                   // points per component root
+  const unsigned long long *largest = nullptr; // size << 32 | label, of sizes >= kSitOutMin
+  const int *roots = nullptr;                  // components (of real points)
+  const int *points = nullptr;                 // points
+  const int *rootOfTile = nullptr;             // null: one instance, root node 0
+  bool everyone = false;                       // no component sits out
+
+  __device__ __forceinline__ int instanceOf(int pos) const {
+    return rootOfTile ? rootOfTile[pos / kTile] : 0;
+  }
+  __device__ __forceinline__ bool sitsOut(int c) const {
+    if (everyone)
+      return false;
+    const int inst = instanceOf(c), count = roots[inst];
+    if (count <= 1)
+      return true;
+    const int s = size[c];
+    return s >= kSitOutMin && ((int)(uint32_t)largest[inst] == c ||
+                               (long long)s * count > 2LL * points[inst]);
+  }
+};
+
+// Every point a component of its own; padding slots have size 0. One thread
+// per position; the points of an instance are counted warp by warp (a warp's
+// positions lie in one tile).
+static __global__ void initComponents(const int *__restrict__ order, int n,
+                                      const int *__restrict__ rootOfTile, int *__restrict__ comp,
+                                      int *__restrict__ size, int *__restrict__ points,
+                                      int *__restrict__ roots) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n)
-    a[i] = i;
+  const bool real = i < n && order[i] >= 0;
+  if (i < n) {
+    comp[i] = i;
+    size[i] = real;
+  }
+  const unsigned bits = __ballot_sync(0xffffffffu, real);
+  if ((threadIdx.x & 31) == 0 && bits) {
+    const int inst = rootOfTile ? rootOfTile[i / kTile] : 0;
+    atomicAdd(&points[inst], __popc(bits));
+    atomicAdd(&roots[inst], __popc(bits));
+  }
 }
 
-static __global__ void fillU32(unsigned int *a, unsigned int v, int n) {
+// Clears the round's per-component results and counters[1..2], and finds each
+// instance's largest component (`largest` was zeroed by the last round).
+static __global__ void startRound(const int *__restrict__ comp, const int *__restrict__ size,
+                                  const int *__restrict__ rootOfTile, int n,
+                                  unsigned int *__restrict__ compBest,
+                                  unsigned long long *__restrict__ compKey,
+                                  unsigned int *__restrict__ compV,
+                                  unsigned long long *__restrict__ largest,
+                                  int *__restrict__ counters) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n)
-    a[i] = v;
+  if (i >= n)
+    return;
+  compBest[i] = 0x7f800000u;
+  compKey[i] = kEmptyKey;
+  compV[i] = 0xffffffffu;
+  if (i == 0)
+    counters[1] = counters[2] = 0;
+  if (comp[i] == i && size[i] >= kSitOutMin)
+    atomicMax(&largest[rootOfTile ? rootOfTile[i / kTile] : 0],
+              ((unsigned long long)(unsigned int)size[i] << 32) | (unsigned int)i);
 }
 
-// The screened pass's per-tile metadata of a round: [orig, comp, value] x
-// 128 slots per tile (PassParams::packedMeta); slots past n hold -1, 0, 0.
-static __global__ void packMeta(const int *__restrict__ order, const int *__restrict__ comp,
-                                const float *__restrict__ value, int n, int numTiles,
-                                int *__restrict__ packed) {
+constexpr float kNoSearch = -1.0f;
+
+// What a row already knows at a round's start. Its lightest known edge to
+// another component (key order: weight, original index): last round's answer
+// if that still leaves, and with k-NN lists the list's members of other
+// components. A member at distance v weighs w = v (single linkage) or
+// max(core_i, core_j, v) (mutual reachability, alpha 1), the bits that the
+// pass computes (fmaxf is exact). Every point outside the list lies at the
+// k-th distance or beyond, hence weighs at least kth = the k-th distance (it
+// is at least core_i). So the known edge is the row's answer when it weighs
+// less than kth, or exactly kth with no point outside the list tying it, or
+// when the list holds every point; such a row is settled. bound[i] <- the
+// least weight an unknown edge can have, kNoSearch for rows that need no
+// search (settled, of a component sitting out, padding). The known edge goes
+// to nearest (the answer unless the pass finds better) and to seed (the pass's
+// starting key), and its weight into the component's best.
+template <bool kMutual>
+static __global__ void seedRows(KnnLists knn, const float *__restrict__ core,
+                                const int *__restrict__ order, const int *__restrict__ rank,
+                                const int *__restrict__ comp, Participation who,
+                                unsigned long long *__restrict__ seed,
+                                unsigned long long *__restrict__ nearest,
+                                unsigned int *__restrict__ compBest, float *__restrict__ bound,
+                                int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n)
+    return;
+  const int c = comp[i];
+  if (order[i] < 0 || who.sitsOut(c)) {
+    seed[i] = nearest[i] = kEmptyKey;
+    bound[i] = kNoSearch;
+    return;
+  }
+  const float ci = kMutual ? core[i] : 0.0f;
+  unsigned long long best = nearest[i];
+  if (best != kEmptyKey && comp[rank[keyIndex(best)]] == c)
+    best = kEmptyKey;
+  float least = ci;
+  bool settled = false;
+  if (knn.pos) {
+    for (int e = 0; e < knn.k; ++e) {
+      const float v = knn.val[knnSlot(i, e, knn.k)];
+      // +inf: the list holds every point; heavier entries cannot win.
+      if (!(v < INFINITY) || (best != kEmptyKey && v > keyWeight(best)))
+        break;
+      const int j = knn.pos[knnSlot(i, e, knn.k)];
+      if (comp[j] == c)
+        continue;
+      const unsigned long long key =
+          packKey(kMutual ? fmaxf(fmaxf(ci, core[j]), v) : v, (uint32_t)order[j]);
+      best = key < best ? key : best;
+    }
+    least = knn.val[knnSlot(i, knn.k - 1, knn.k)];
+    const float w = best == kEmptyKey ? INFINITY : keyWeight(best);
+    settled = !(least < INFINITY) || w < least || (w == least && knn.tie[i] == 0);
+  }
+  if (best != kEmptyKey) {
+    const unsigned int bits = (unsigned int)(best >> 32);
+    if (bits < __ldcg(&compBest[c]))
+      atomicMin(&compBest[c], bits);
+  }
+  nearest[i] = best;
+  seed[i] = best;
+  bound[i] = settled ? kNoSearch : least;
+}
+
+// flag[i] <- whether row i searches: it may know too little (bound >= 0), and
+// an edge it does not know could still be its component's lightest or tie it.
+// Also the screened pass's per-tile metadata of the round (packed, may be
+// null): [orig, comp, value] x 128 slots per tile; slots past n hold -1, 0, 0.
+static __global__ void chooseRows(const float *__restrict__ bound,
+                                  const unsigned int *__restrict__ compBest,
+                                  const int *__restrict__ order, const int *__restrict__ comp,
+                                  const float *__restrict__ value, int n, int numTiles,
+                                  unsigned char *__restrict__ flag, int *__restrict__ packed) {
   const int pos = blockIdx.x * blockDim.x + threadIdx.x;
   if (pos >= numTiles * kTile)
     return;
-  int *tile = packed + (size_t)(pos / kTile) * 3 * kTile + pos % kTile;
   const bool real = pos < n;
-  tile[0] = real ? order[pos] : -1;
-  tile[kTile] = real ? comp[pos] : 0;
-  tile[2 * kTile] = real && value ? __float_as_int(value[pos]) : 0;
+  if (real && flag) {
+    const float b = bound[pos];
+    flag[pos] = b >= 0.0f && b <= bitsFloat(compBest[comp[pos]]);
+  }
+  if (packed) {
+    int *tile = packed + (size_t)(pos / kTile) * 3 * kTile + pos % kTile;
+    tile[0] = real ? order[pos] : -1;
+    tile[kTile] = real ? comp[pos] : 0;
+    tile[2 * kTile] = real && value ? __float_as_int(value[pos]) : 0;
+  }
 }
 
-// compBest[comp[i]] <- min over i of last round's edge weights that leave
-// the (new) component of i.
-static __global__ void seedComponentBest(const unsigned long long *__restrict__ nearest,
-                                  const int *__restrict__ rank, const int *__restrict__ comp,
-                                  unsigned int *__restrict__ compBest, int n) {
+// Learned radius: rows of components that sit the round out are not proposed
+// (radius -1); counts the others.
+static __global__ void proposeRows(const int *__restrict__ order, const int *__restrict__ comp,
+                                   Participation who, int n, float *__restrict__ radius,
+                                   unsigned long long *__restrict__ proposed) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n)
-    return;
-  const unsigned long long key = nearest[i];
-  if (key == kEmptyKey)
-    return;
-  const int j = rank[keyIndex(key)];
-  if (comp[j] != comp[i])
-    atomicMin(&compBest[comp[i]], (unsigned int)(key >> 32));
-}
-
-// Seeds of a round from HDBSCAN's k-NN lists (mutual reachability, alpha
-// 1). A list member j of row i lies within core_i, so the edge (i, j) weighs
-// max(core_i, core_j) (fmaxf is exact: the pass computes the same bits).
-// Per row: seed = the lightest such edge to another component, under the
-// key order (weight, original index), and its weight goes into the
-// component's best (a real edge: a valid bound). The seed is the row's final
-// answer when it weighs core_i and no point outside the list ties the k-th
-// distance: every point outside the list is then farther than core_i, so its
-// edge weighs more than core_i, the least any edge of row i can weigh. Such a
-// row is settled: its answer goes to nearest now and the pass skips it.
-static __global__ void seedFromKnn(const int *__restrict__ knnPos, const int *__restrict__ knnTie,
-                                   int k, const float *__restrict__ core,
-                                   const int *__restrict__ order, const int *__restrict__ comp,
-                                   unsigned long long *__restrict__ seed,
-                                   unsigned long long *__restrict__ nearest,
-                                   unsigned int *__restrict__ compBest, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n)
-    return;
-  if (order[i] < 0) {
-    seed[i] = kEmptyKey;
-    return;
+  bool takes = i < n && order[i] >= 0;
+  if (takes && who.sitsOut(comp[i])) {
+    radius[i] = -1.0f;
+    takes = false;
   }
-  const float ci = core[i];
-  const int c = comp[i];
-  unsigned long long best = kEmptyKey;
-  const int *list = knnPos + (size_t)i * k;
-  for (int e = 0; e < k; ++e) {
-    const int j = list[e];
-    if (j < 0 || j == i || comp[j] == c)
-      continue;
-    const unsigned long long key = packKey(fmaxf(ci, core[j]), (uint32_t)order[j]);
-    best = key < best ? key : best;
-  }
-  if (best == kEmptyKey) {
-    seed[i] = kEmptyKey;
-    return;
-  }
-  atomicMin(&compBest[c], (unsigned int)(best >> 32));
-  const bool settled = keyWeight(best) == ci && knnTie[i] == 0;
-  seed[i] = settled ? (best | kSettledKey) : best;
-  if (settled)
-    nearest[i] = best;
+  const unsigned bits = __ballot_sync(0xffffffffu, takes);
+  if ((threadIdx.x & 31) == 0 && bits)
+    atomicAdd(proposed, (unsigned long long)__popc(bits));
 }
 
 static __global__ void componentKeyPass1(const unsigned long long *__restrict__ nearest,
@@ -187,8 +289,13 @@ static __global__ void hookComponents(const int *__restrict__ comp, const int *_
                                const unsigned int *__restrict__ compV, int *__restrict__ parent,
                                int *__restrict__ edgeU, int *__restrict__ edgeV,
                                float *__restrict__ edgeW, int *__restrict__ counters,
-                               int edgeCapacity, int n) {
+                               int edgeCapacity, int n, unsigned long long *__restrict__ largest,
+                               int *__restrict__ roots, int numNodes) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r < numNodes) { // counted anew by finishRoots and the next startRound
+    largest[r] = 0;
+    roots[r] = 0;
+  }
   if (r >= n || comp[r] != r)
     return;
   const unsigned long long k1 = compKey[r];
@@ -215,22 +322,49 @@ static __global__ void hookComponents(const int *__restrict__ comp, const int *_
   }
 }
 
-static __global__ void jumpParents(const int *__restrict__ comp, int *__restrict__ parent, int n) {
+// Follows each root's parent chain up to kHops steps and points the root at
+// its end. Other threads shorten the chain meanwhile, which only skips
+// ancestors, so L launches reach at least kHops^L steps up.
+constexpr int kHops = 16;
+
+static __global__ void jumpParents(const int *__restrict__ comp, int *parent, int n) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n || comp[r] != r)
     return;
-  parent[r] = parent[parent[r]];
+  volatile int *up = parent;
+  int at = up[r];
+  for (int h = 0; h < kHops; ++h) {
+    const int next = up[at];
+    if (next == at)
+      break;
+    at = next;
+  }
+  up[r] = at;
 }
 
-static __global__ void countRoots(const int *__restrict__ comp, const int *__restrict__ parent,
-                           int *__restrict__ counters, int n) {
+// Counts the new components (counters[1]; per instance, padding slots left
+// out, roots) and adds the absorbed components' sizes to their roots'.
+static __global__ void finishRoots(const int *__restrict__ comp, const int *__restrict__ parent,
+                                   const int *__restrict__ order,
+                                   const int *__restrict__ rootOfTile, int *__restrict__ size,
+                                   int *__restrict__ roots, int *__restrict__ counters, int n) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n || comp[r] != r)
-    return;
-  if (parent[r] == r)
-    atomicAdd(&counters[1], 1);
-  if (parent[parent[r]] != parent[r])
-    atomicAdd(&counters[2], 1); // not fully jumped (would be a bug)
+  const bool old = r < n && comp[r] == r;
+  const int up = old ? parent[r] : -1;
+  const bool root = old && up == r, real = root && order[r] >= 0;
+  const unsigned allBits = __ballot_sync(0xffffffffu, root);
+  const unsigned bits = __ballot_sync(0xffffffffu, real);
+  if ((threadIdx.x & 31) == 0) {
+    if (allBits)
+      atomicAdd(&counters[1], __popc(allBits));
+    if (bits)
+      atomicAdd(&roots[rootOfTile ? rootOfTile[r / kTile] : 0], __popc(bits));
+  }
+  if (old && !root) {
+    atomicAdd(&size[up], size[r]);
+    if (parent[up] != up)
+      atomicAdd(&counters[2], 1); // not fully jumped (would be a bug)
+  }
 }
 
 static __global__ void relabel(int *__restrict__ comp, const int *__restrict__ parent, int n) {
@@ -255,24 +389,42 @@ int boruvkaMst(SpatialIndex &index, const Metric &metric, const Weight &weight, 
   if (n < 2 || !st.ok())
     return st.code;
 
-  DeviceBuffer<int> comp, parent, counters, error;
-  DeviceBuffer<unsigned long long> nearest, compKey, tiles;
+  const int numNodes = index.topo.numNodes;
+  const int *rootOfTile = index.numInstances > 1 ? index.rootOfTile.get() : nullptr;
+  DeviceBuffer<int> comp, parent, counters, size, instanceRoots, instancePoints;
+  DeviceBuffer<unsigned long long> nearest, compKey, tiles, seed, largest;
   DeviceBuffer<unsigned int> compBest, compV;
+  DeviceBuffer<float> bound;
+  DeviceBuffer<unsigned char> flag;
   CUHC_TRY(st, comp.allocate(paddedToTiles(n), stream));
   CUHC_TRY(st, parent.allocate(n, stream));
+  // Edges so far, roots, unjumped parents, the passes' error word.
   CUHC_TRY(st, counters.allocate(4, stream));
-  CUHC_TRY(st, error.allocate(1, stream));
+  CUHC_TRY(st, size.allocate(n, stream));
+  CUHC_TRY(st, instanceRoots.allocate(numNodes, stream));
+  CUHC_TRY(st, instancePoints.allocate(numNodes, stream));
+  CUHC_TRY(st, largest.allocate(numNodes, stream));
   CUHC_TRY(st, nearest.allocate(n, stream));
+  CUHC_TRY(st, seed.allocate(n, stream));
+  CUHC_TRY(st, bound.allocate(n, stream));
+  CUHC_TRY(st, flag.allocate(n, stream));
   CUHC_TRY(st, compKey.allocate(n, stream));
   CUHC_TRY(st, tiles.allocate(1, stream));
   CUHC_TRY(st, compBest.allocate(n, stream));
   CUHC_TRY(st, compV.allocate(n, stream));
   if (!st.ok())
     return st.code;
-  iotaKernel<<<blocks(n), 256, 0, stream>>>(comp.get(), n); noteLaunch();
+  CUHC_TRY(st, cudaMemsetAsync(instanceRoots.get(), 0, instanceRoots.bytes(), stream));
+  CUHC_TRY(st, cudaMemsetAsync(instancePoints.get(), 0, instancePoints.bytes(), stream));
+  CUHC_TRY(st, cudaMemsetAsync(largest.get(), 0, largest.bytes(), stream));
   CUHC_TRY(st, cudaMemsetAsync(nearest.get(), 0xff, n * sizeof(unsigned long long), stream));
-  CUHC_TRY(st, cudaMemsetAsync(error.get(), 0, sizeof(int), stream));
+  CUHC_TRY(st, cudaMemsetAsync(counters.get(), 0, 4 * sizeof(int), stream));
   CUHC_TRY(st, cudaMemsetAsync(tiles.get(), 0, sizeof(unsigned long long), stream));
+  initComponents<<<blocks(n), 256, 0, stream>>>(index.order.get(), n, rootOfTile, comp.get(),
+                                                size.get(), instancePoints.get(),
+                                                instanceRoots.get());
+  noteLaunch();
+  CUHC_TRY(st, cudaGetLastError());
 
   PassParams p{};
   p.tiled = index.tiled.get();
@@ -294,32 +446,27 @@ int boruvkaMst(SpatialIndex &index, const Metric &metric, const Weight &weight, 
   p.nearest = nearest.get();
   p.compBest = compBest.get();
   p.tilesComputed = tiles.get();
-  p.error = error.get();
+  p.error = counters.get() + 3;
   p.screenStats = screenCounters();
   p.screenAudit = screenAuditWords();
-  p.rootOfTile = index.numInstances > 1 ? index.rootOfTile.get() : nullptr;
+  p.rootOfTile = rootOfTile;
 
   const bool screened = useScreen<Metric>(index.d, 0) && screenDataOk<Metric>(index);
   DeviceBuffer<int> packed;
   if (screened)
     CUHC_TRY(st, packed.allocate((size_t)index.numTiles * 3 * kTile, stream));
-  // Seeds from the k-NN lists (mutual reachability with alpha 1 only: there
-  // a list edge's weight needs no distance).
-  bool seeds = false;
-  if constexpr (std::is_same<Weight, MutualReachWeight>::value)
-    seeds = knn && knn->pos && weight.alpha == 1.0f && index.numInstances == 1;
-  DeviceBuffer<unsigned long long> seed;
-  if (seeds)
-    CUHC_TRY(st, seed.allocate(n, stream));
   int numComponents = n, totalEdges = 0, rounds = 0;
   unsigned long long tilesSoFar = 0;
   int hostCounters[4];
   // Each instance of a batch ends as one component; padding slots stay
   // components of their own.
   const int finalComponents = index.numInstances + index.numPads;
-  int maxJumps = 1;
-  while ((1 << maxJumps) < n)
-    ++maxJumps;
+  auto jumpsFor = [](int components) {
+    int launches = 1;
+    for (long long reach = kHops; reach < components; reach *= kHops)
+      ++launches;
+    return launches;
+  };
   // Radius proposal (single linkage, one instance, 16 features, a model
   // loaded) or training-row logging: per-round features of every position.
   const RadiusModel model = currentRadiusModel();
@@ -328,6 +475,33 @@ int boruvkaMst(SpatialIndex &index, const Metric &metric, const Weight &weight, 
                          index.numInstances == 1;
   const bool logRows = plainWeight && radiusLog && index.d == kRadiusDims &&
                        index.numInstances == 1;
+  // Lists give edges whose weight is known without the distance formula:
+  // plain weights, and mutual reachability with alpha 1.
+  KnnLists lists;
+  bool listsUsable = plainWeight;
+  if constexpr (std::is_same<Weight, MutualReachWeight>::value)
+    listsUsable = weight.alpha == 1.0f;
+  if (knn && listsUsable && !logRows)
+    lists = *knn;
+  Participation who;
+  who.size = size.get();
+  who.largest = largest.get();
+  who.roots = instanceRoots.get();
+  who.points = instancePoints.get();
+  who.rootOfTile = rootOfTile;
+  // The rows that search are a scattered few in most rounds. Packed into row
+  // tiles of their own they need a fraction of the blocks, and few row tiles
+  // can be split over the columns (blockWork); but a packed row tile spans
+  // many tiles' worth of space, so its box excludes less. Packing pays where
+  // boxes exclude little anyway, which the list pass has just measured: the
+  // share of tile pairs it computed. Rounds' passes in ms, in place against
+  // packed: share 1.00 (300,000 x 32 normal) 11.1 / 0.3; 0.93 (50,001 x 50
+  // blobs, HDBSCAN) 41.7 / 29.4; 0.79 (batch, 32 features) 15.5 / 12.9; 0.47
+  // (batch, 8 features) 2.5 / 3.4; 0.48 (500,000 x 16) 61.7 / 58.4; 0.25
+  // (100,000 x 8, HDBSCAN) 1.02 / 1.22; 0.08 (1,000,000 x 8, HDBSCAN) 15.1 /
+  // 12.9; 0.04 (batch, 2 features) 3.1 / 9.6.
+  const bool packRows = lists.pos && lists.tilesSearched > 0.5 * index.fullTilePairs();
+  who.everyone = logRows; // training rows want every row's answer, every round
   DeviceBuffer<float> features, prediction, radius, targets;
   DeviceBuffer<int> compSize;
   DeviceBuffer<unsigned long long> certified;
@@ -337,8 +511,9 @@ int boruvkaMst(SpatialIndex &index, const Metric &metric, const Weight &weight, 
     CUHC_TRY(st, prediction.allocate(n, stream));
     CUHC_TRY(st, radius.allocate(n, stream));
     CUHC_TRY(st, targets.allocate(n, stream));
-    CUHC_TRY(st, certified.allocate(4, stream)); // certified rows, then [mark, capped, fallback]
-    CUHC_TRY(st, cudaMemsetAsync(certified.get(), 0, 4 * sizeof(unsigned long long), stream));
+    // Certified rows, [mark, capped, fallback], proposed rows.
+    CUHC_TRY(st, certified.allocate(5, stream));
+    CUHC_TRY(st, cudaMemsetAsync(certified.get(), 0, 5 * sizeof(unsigned long long), stream));
   }
   auto enqueueFeatures = [&](int round) {
     StatusChain fs;
@@ -355,7 +530,6 @@ int boruvkaMst(SpatialIndex &index, const Metric &metric, const Weight &weight, 
     return fs.code;
   };
   std::mt19937_64 logRng(radiusLog ? radiusLog->seed : 0);
-  unsigned long long proposedRows = 0;
 
   // One round, enqueued on the stream with no host work: counters[0] counts
   // every edge so far (edges are written at absolute slots), counters[1..2]
@@ -363,43 +537,58 @@ int boruvkaMst(SpatialIndex &index, const Metric &metric, const Weight &weight, 
   auto enqueueRound = [&](bool first, int jumps, bool timed) {
     StatusChain rs;
     CUHC_TRY(rs, index.updatePurity(comp.get()));
-    fillU32<<<blocks(n), 256, 0, stream>>>(compBest.get(), 0x7f800000u, n); noteLaunch();
-    if (!first) {
-      seedComponentBest<<<blocks(n), 256, 0, stream>>>(nearest.get(), index.rank.get(),
-                                                       comp.get(), compBest.get(), n);
+    startRound<<<blocks(n), 256, 0, stream>>>(comp.get(), size.get(), rootOfTile, n,
+                                              compBest.get(), compKey.get(), compV.get(),
+                                              largest.get(), counters.get());
+    noteLaunch();
+    if (useRadius || logRows)
+      CUHC_TRY(rs, enqueueFeatures(rounds));
+    seedRows<!std::is_same<Weight, PlainWeight>::value><<<blocks(n), 256, 0, stream>>>(
+        lists, weight.value, index.order.get(), index.rank.get(), comp.get(), who, seed.get(),
+        nearest.get(), compBest.get(), bound.get(), n);
+    noteLaunch();
+    p.seedKey = logRows ? nullptr : seed.get();
+    // A first round without lists searches every row; so do training rows.
+    const bool chosen = !logRows && (lists.pos || !first), someRows = chosen && packRows;
+    if (chosen || screened) {
+      chooseRows<<<blocks(index.numTiles * kTile), 256, 0, stream>>>(
+          bound.get(), compBest.get(), index.order.get(), comp.get(), weight.value, n,
+          index.numTiles, chosen ? flag.get() : nullptr, screened ? packed.get() : nullptr);
       noteLaunch();
-    }
-    if constexpr (std::is_same<Weight, MutualReachWeight>::value) {
-      if (seeds) {
-        seedFromKnn<<<blocks(n), 256, 0, stream>>>(knn->pos, knn->tie, knn->k, weight.value,
-                                                   index.order.get(), comp.get(), seed.get(),
-                                                   nearest.get(), compBest.get(), n);
-        noteLaunch();
-        p.seedKey = seed.get();
-      }
-    }
-    if (screened) {
-      packMeta<<<blocks(index.numTiles * kTile), 256, 0, stream>>>(
-          index.order.get(), comp.get(), weight.value, n, index.numTiles, packed.get());
-      noteLaunch();
-      p.packedMeta = packed.get();
+      p.packedMeta = screened ? packed.get() : nullptr;
     }
     CUHC_TRY(rs, cudaGetLastError());
     p.singletons = first;
     p.radius = nullptr;
-    // Heaviest row tiles first: by the last pass's work (boxes before any).
-    CUHC_TRY(rs, index.orderTiles(!index.tileWorkValid, true));
-    p.tileOrder = index.tileOrder.get();
-    p.tileWork = index.tileWork.get();
-    if (useRadius || logRows)
-      CUHC_TRY(rs, enqueueFeatures(rounds));
+    p.active = chosen ? flag.get() : nullptr;
+    // Heaviest row tiles first: by the last full pass's work (boxes before any).
+    if (someRows) {
+      bool ordered = false;
+      CUHC_TRY(rs, index.selectRows(flag.get(), comp.get(),
+                                    index.hasMinValues ? weight.value : nullptr, &ordered));
+      p.rowPos = index.rowPos.get();
+      p.rowTiles = index.rowTiles.get();
+      p.rowTiled = index.rowTiled.get();
+      p.rowBoxLow = index.rowBoxLow.get();
+      p.rowBoxHigh = index.rowBoxHigh.get();
+      p.rowMinValue = index.rowMinValue.get();
+      p.rowPure = index.rowPure.get();
+      p.tileOrder = ordered ? index.tileOrder.get() : nullptr;
+      p.tileWork = nullptr;
+    } else if (index.orderMatters()) {
+      CUHC_TRY(rs, index.orderTiles(!index.tileWorkValid, true));
+      p.tileOrder = index.tileOrder.get();
+      p.tileWork = index.tileWork.get();
+    }
     if (useRadius) {
       CUHC_TRY(rs, mlpForward(model.params, features.get(), n, prediction.get(), stream));
       radius_detail::radiusFromPrediction<<<blocks(n), 256, 0, stream>>>(
           prediction.get(), index.order.get(), n, model.offset, radius.get());
       noteLaunch();
+      proposeRows<<<blocks(n), 256, 0, stream>>>(index.order.get(), comp.get(), who, n,
+                                                 radius.get(), certified.get() + 4);
+      noteLaunch();
       p.radius = radius.get();
-      proposedRows += (unsigned long long)index.numPoints;
       radius_detail::radiusTileStep<<<1, 1, 0, stream>>>(tiles.get(), 0, certified.get() + 1);
       noteLaunch();
     }
@@ -461,22 +650,24 @@ int boruvkaMst(SpatialIndex &index, const Metric &metric, const Weight &weight, 
         radiusLog->targets.push_back(ht[i]);
       }
     }
-    index.tileWorkValid = true;
-    CUHC_TRY(rs, cudaMemsetAsync(compKey.get(), 0xff, n * sizeof(unsigned long long), stream));
-    CUHC_TRY(rs, cudaMemsetAsync(compV.get(), 0xff, n * sizeof(unsigned int), stream));
-    CUHC_TRY(rs, cudaMemsetAsync(counters.get() + 1, 0, 2 * sizeof(int), stream));
+    if (!someRows)
+      index.tileWorkValid = true;
     componentKeyPass1<<<blocks(n), 256, 0, stream>>>(nearest.get(), index.order.get(), comp.get(),
                                                      compKey.get(), n); noteLaunch();
     componentKeyPass2<<<blocks(n), 256, 0, stream>>>(nearest.get(), index.order.get(), comp.get(),
                                                      compKey.get(), compV.get(), n); noteLaunch();
     hookComponents<<<blocks(n), 256, 0, stream>>>(
         comp.get(), index.rank.get(), compKey.get(), compV.get(), parent.get(), edges.u.get(),
-        edges.v.get(), edges.w.get(), counters.get(), n - 1, n); noteLaunch();
-    for (int jmp = 0; jmp <= jumps; ++jmp) {
+        edges.v.get(), edges.w.get(), counters.get(), n - 1, n, largest.get(),
+        instanceRoots.get(), numNodes); noteLaunch();
+    for (int jmp = 0; jmp < jumps; ++jmp) {
       jumpParents<<<blocks(n), 256, 0, stream>>>(comp.get(), parent.get(), n);
       noteLaunch();
     }
-    countRoots<<<blocks(n), 256, 0, stream>>>(comp.get(), parent.get(), counters.get(), n); noteLaunch();
+    finishRoots<<<blocks(n), 256, 0, stream>>>(comp.get(), parent.get(), index.order.get(),
+                                               rootOfTile, size.get(), instanceRoots.get(),
+                                               counters.get(), n);
+    noteLaunch();
     relabel<<<blocks(n), 256, 0, stream>>>(comp.get(), parent.get(), n); noteLaunch();
     CUHC_TRY(rs, cudaGetLastError());
     return rs.code;
@@ -487,12 +678,11 @@ int boruvkaMst(SpatialIndex &index, const Metric &metric, const Weight &weight, 
   const bool useGraph = index.numInstances > 1 && !timingEnabled();
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graphExec = nullptr;
-  CUHC_TRY(st, cudaMemsetAsync(counters.get(), 0, 4 * sizeof(int), stream));
   while (st.ok() && numComponents > finalComponents) {
     if (useGraph && rounds > 0) {
       if (!graphExec) {
         CUHC_TRY(st, cudaStreamBeginCapture(stream, cudaStreamCaptureModeRelaxed));
-        const int captured = enqueueRound(false, maxJumps, false);
+        const int captured = enqueueRound(false, jumpsFor(n), false);
         const cudaError_t ended = cudaStreamEndCapture(stream, &graph);
         CUHC_TRY(st, captured);
         CUHC_TRY(st, ended);
@@ -502,22 +692,16 @@ int boruvkaMst(SpatialIndex &index, const Metric &metric, const Weight &weight, 
       }
       CUHC_TRY(st, cudaGraphLaunch(graphExec, stream));
     } else {
-      int jumps = 1;
-      while ((1 << jumps) < numComponents)
-        ++jumps;
-      CUHC_TRY(st, enqueueRound(rounds == 0, jumps, true));
+      CUHC_TRY(st, enqueueRound(rounds == 0, jumpsFor(numComponents), true));
     }
-    int passError = 0;
     CUHC_TRY(st, cudaMemcpyAsync(hostCounters, counters.get(), 4 * sizeof(int),
                                  cudaMemcpyDeviceToHost, stream));
-    CUHC_TRY(st, cudaMemcpyAsync(&passError, error.get(), sizeof(int), cudaMemcpyDeviceToHost,
-                                 stream));
     CUHC_TRY(st, cudaStreamSynchronize(stream));
     if (!st.ok())
       break;
     ++rounds;
-    if (passError != 0) {
-      st(passError);
+    if (hostCounters[3] != 0) {
+      st(hostCounters[3]);
       break;
     }
     const int added = hostCounters[0] - totalEdges;
@@ -537,23 +721,19 @@ int boruvkaMst(SpatialIndex &index, const Metric &metric, const Weight &weight, 
     }
   }
   if (useRadius) {
-    unsigned long long counts[4] = {};
+    unsigned long long counts[5] = {};
     cudaMemcpyAsync(counts, certified.get(), sizeof(counts), cudaMemcpyDeviceToHost, stream);
     cudaStreamSynchronize(stream);
-    addRadiusStats(proposedRows, counts[0], counts[2], counts[3]);
+    addRadiusStats(counts[4], counts[0], counts[2], counts[3]);
   }
   if (graphExec)
     cudaGraphExecDestroy(graphExec);
   if (graph)
     cudaGraphDestroy(graph);
-  int err = 0;
   unsigned long long tileCount = 0;
-  CUHC_TRY(st, cudaMemcpyAsync(&err, error.get(), sizeof(int), cudaMemcpyDeviceToHost, stream));
   CUHC_TRY(st, cudaMemcpyAsync(&tileCount, tiles.get(), sizeof(tileCount),
                                cudaMemcpyDeviceToHost, stream));
   CUHC_TRY(st, cudaStreamSynchronize(stream));
-  if (err)
-    st(err);
   edges.count = totalEdges;
   if (stats) {
     stats->tilesComputed += tileCount;
@@ -566,8 +746,8 @@ int boruvkaMst(SpatialIndex &index, const Metric &metric, const Weight &weight, 
 
 template <class Metric>
 int coreDistances(SpatialIndex &index, const Metric &metric, int k, bool prune, float *core,
-                  PassStats *stats, cudaStream_t stream, const int *coreRank, int *knnPos,
-                  int *knnTie) {
+                  PassStats *stats, cudaStream_t stream, const int *coreRank,
+                  KnnLists *lists, bool rounds) {
   StatusChain st;
   DeviceBuffer<unsigned long long> tiles;
   DeviceBuffer<int> error;
@@ -597,11 +777,16 @@ int coreDistances(SpatialIndex &index, const Metric &metric, int k, bool prune, 
   p.core = core;
   p.k = k;
   p.coreRank = coreRank;
-  p.knnPos = knnPos;
-  p.knnTie = knnTie;
-  CUHC_TRY(st, index.orderTiles(!index.tileWorkValid));
-  p.tileOrder = index.tileOrder.get();
-  p.tileWork = index.tileWork.get();
+  if (lists) {
+    p.knnPos = lists->pos;
+    p.knnVal = lists->val;
+    p.knnTie = lists->tie;
+  }
+  if (index.orderMatters()) {
+    CUHC_TRY(st, index.orderTiles(!index.tileWorkValid));
+    p.tileOrder = index.tileOrder.get();
+    p.tileWork = index.tileWork.get();
+  }
   p.tilesComputed = tiles.get();
   p.error = error.get();
   p.screenStats = screenCounters();
@@ -610,10 +795,13 @@ int coreDistances(SpatialIndex &index, const Metric &metric, int k, bool prune, 
   {
     const bool screened =
         useScreen<Metric>(index.d, k) && screenDataOk<Metric>(index);
-    const ScreenShape shape =
-        screened ? tunedScreenShape<Metric>(index, metric, k, core, stream) : ScreenShape{};
+    const ScreenShape shape = screened && !rounds
+                                  ? tunedScreenShape<Metric>(index, metric, k, core, stream)
+                                  : ScreenShape{};
     ScreenShapeScope shapeScope(shape);
-    PassTimer timer(screened ? kTimerScreenKnnPass : kTimerKnnPass, stream);
+    PassTimer timer(rounds ? (screened ? kTimerScreenPass : kTimerNearestPass)
+                           : (screened ? kTimerScreenKnnPass : kTimerKnnPass),
+                    stream);
     if (screened)
       CUHC_TRY(st, (launchScreen<Metric, PlainWeight, true>(p, metric, PlainWeight{}, index.kc,
                                                             stream)));
@@ -635,6 +823,8 @@ int coreDistances(SpatialIndex &index, const Metric &metric, int k, bool prune, 
   CUHC_TRY(st, cudaStreamSynchronize(stream));
   if (err)
     st(err);
+  if (lists)
+    lists->tilesSearched = (double)tileCount;
   if (stats) {
     stats->tilesComputed += tileCount;
     stats->tilesTotal += (unsigned long long)index.numTiles * index.numTiles;

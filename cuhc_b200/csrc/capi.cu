@@ -42,6 +42,13 @@ constexpr int kMaxListK = 256;
 // Largest k whose lists are kept for the Borůvka seeds (values and positions
 // in shared memory).
 constexpr int kMaxKeptListK = 64;
+// Entries of the lists that single linkage keeps (the point itself included).
+// Longer lists settle more rows but widen every row's search radius. Odd, so
+// that the rows' lists spread over the shared-memory banks. Whole calls in ms
+// for 5 / 9 / 13 / 17 entries: 300,000 x 32 normal 82.7 / 77.8 / 75.7 / 78.4,
+// 500,000 x 16 anisotropic 146 / 138 / 145 / 155, 20,000 x 32 6.9 / 6.2 / 6.0
+// / 6.1 (packed rows, one block per row tile).
+constexpr int kSingleListK = 9;
 
 std::atomic<int> gPruneMode{kPruneAuto};
 std::mutex gStatsMutex;
@@ -130,7 +137,19 @@ int singleLinkageMst(const float *devPoints, int n, int d, const Metric &m, doub
   CUHC_TRY(st, index.build(devPoints, n, d, prune, s));
   DeviceEdges edges;
   PassStats stats;
-  CUHC_TRY(st, (boruvkaMst<Metric, PlainWeight>(index, m, PlainWeight{}, prune, edges, &stats, s)));
+  // The first round's search keeps every point's nearest few (itself
+  // included): the later rounds then know most rows' answers, or that they
+  // cannot matter, without a search.
+  const int k = std::min(kSingleListK, n);
+  KnnListBuffers lists;
+  DeviceBuffer<float> kth;
+  CUHC_TRY(st, lists.allocate(n, k, s));
+  CUHC_TRY(st, kth.allocate(paddedToTiles(n), s));
+  KnnLists knn = lists.lists(k);
+  CUHC_TRY(st, coreDistances<Metric>(index, m, k, prune, kth.get(), &stats, s, nullptr, &knn,
+                                     true));
+  CUHC_TRY(st, (boruvkaMst<Metric, PlainWeight>(index, m, PlainWeight{}, prune, edges, &stats, s,
+                                                nullptr, &knn)));
   HostEdges sorted;
   CUHC_TRY(st, sortEdgesToPinned(edges, edges.count, s, sorted));
   if (st.ok() && sorted.count != n - 1)
@@ -157,30 +176,25 @@ int hdbscanTree(const float *devPoints, int n, int d, const Metric &m, int minSa
   // that fit shared memory twice over.
   const bool radix = coreMethod == kCoreRadix || minSamples > kMaxListK;
   const bool keepLists = !radix && alpha == 1.0f && minSamples <= kMaxKeptListK && n > 1;
-  DeviceBuffer<int> knnPos, knnTie;
-  if (keepLists) {
-    CUHC_TRY(st, knnPos.allocate((size_t)n * minSamples, s));
-    CUHC_TRY(st, knnTie.allocate(n, s));
-  }
+  KnnListBuffers lists;
+  if (keepLists)
+    CUHC_TRY(st, lists.allocate(n, minSamples, s));
+  KnnLists knn = lists.lists(minSamples);
   // Radix select when asked for, or when the per-row lists would not fit
   // shared memory (the reference's Auto picks radix above k = 64).
   if (radix)
     CUHC_TRY(st, coreDistancesRadix<Metric>(index, m, minSamples, core.get(), s));
   else
     CUHC_TRY(st, coreDistances<Metric>(index, m, minSamples, prune, core.get(), &stats, s,
-                                       nullptr, knnPos.get(), knnTie.get()));
+                                       nullptr, keepLists ? &knn : nullptr));
   CUHC_TRY(st, index.updateMinValues(core.get()));
   DeviceEdges edges;
   MutualReachWeight weight;
   weight.value = core.get();
   weight.alpha = alpha;
-  KnnLists lists;
-  lists.pos = knnPos.get();
-  lists.tie = knnTie.get();
-  lists.k = minSamples;
   if (n > 1)
     CUHC_TRY(st, (boruvkaMst<Metric, MutualReachWeight>(index, m, weight, prune, edges, &stats, s,
-                                                        nullptr, keepLists ? &lists : nullptr)));
+                                                        nullptr, keepLists ? &knn : nullptr)));
   if (hostCore && st.ok()) {
     CUHC_TRY(st, coreOrig.allocate(n, s));
     scatterByOrder<<<(n + 255) / 256, 256, 0, s>>>(core.get(), index.order.get(), coreOrig.get(),
@@ -274,19 +288,28 @@ int batchTrees(const float *devPoints, const std::vector<int> &sizes,
   CUHC_TRY(st, cudaStreamSynchronize(s));
   if (!st.ok())
     return st.code;
-  ScreenOverride screen(tuneScreen(index, m, metricId, std::max(maxK, 1), core.get(), s));
+  // Lists for the rounds, as single calls keep them: of the largest rank, and
+  // at least of the length single linkage keeps.
+  const bool keepLists = maxK <= kMaxKeptListK;
+  const int listK = keepLists ? std::max(maxK, kSingleListK) : maxK;
+  ScreenOverride screen(tuneScreen(index, m, metricId, listK, core.get(), s));
   CUHC_TRY(st, cudaMemsetAsync(core.get(), 0, core.bytes(), s));
   PassStats stats;
+  KnnListBuffers lists;
+  if (keepLists)
+    CUHC_TRY(st, lists.allocate(positions, listK, s));
+  KnnLists knn = lists.lists(listK);
   // Mutual reachability with core 0 is the plain distance (keys clamp at 0),
   // so single-linkage instances (rank 0) share the solve with HDBSCAN ones.
-  if (maxK > 0)
-    CUHC_TRY(st, coreDistances<Metric>(index, m, maxK, true, core.get(), &stats, s, rank.get()));
+  CUHC_TRY(st, coreDistances<Metric>(index, m, listK, true, core.get(), &stats, s, rank.get(),
+                                     keepLists ? &knn : nullptr));
   CUHC_TRY(st, index.updateMinValues(core.get()));
   MutualReachWeight weight;
   weight.value = core.get();
   weight.alpha = 1.0f;
   DeviceEdges edges;
-  CUHC_TRY(st, (boruvkaMst<Metric, MutualReachWeight>(index, m, weight, true, edges, &stats, s)));
+  CUHC_TRY(st, (boruvkaMst<Metric, MutualReachWeight>(index, m, weight, true, edges, &stats, s,
+                                                      nullptr, keepLists ? &knn : nullptr)));
   // Edges sorted by (instance, w, u, v) on the device, in local ids: instance
   // i's n_i - 1 edges at slots offsets[i] - i ...; then every instance's tree
   // on the host threads.

@@ -169,25 +169,91 @@ struct PassParams {
   // computed (null: not recorded).
   const int *tileOrder;
   unsigned int *tileWork;
-  // Knn mode: per position, the positions of its k list entries in
-  // ascending distance (k ints) and a flag set when a point outside the list
-  // lies at exactly the k-th distance (null: not recorded).
+  // Knn mode: per position, the positions and distances of its k list entries
+  // in ascending distance (knnSlot) and a flag set when a point outside the
+  // list lies at exactly the k-th distance (null: not recorded).
   int *knnPos;
+  float *knnVal;
   int *knnTie;
   // Nearest mode: per position an initial best key (a real edge of the row,
-  // kEmptyKey: none); kSettledKey in the index bits marks a key that is
-  // already the row's answer: the row neither searches nor writes (null:
-  // no seeds).
+  // kEmptyKey: none; null: no seeds), and whether the row searches (null: all
+  // do); a row that does not keeps what `nearest` holds.
   const unsigned long long *seedKey;
+  const unsigned char *active;
   // Screened passes: per tile, the original indices, component labels and
   // weight values of its 128 slots packed as [3][128] 32-bit words, so that
   // one bulk copy stages a column tile's metadata (null: three copies from
   // order, component and the weight's value array).
   const int *packedMeta;
+  // Nearest mode over some of the rows: row r of row tile I is the point at
+  // position rowPos[I * kTile + r] (-1: none; a tile's rows come first, so a
+  // tile without a first row is empty and its block leaves at once). The row
+  // tiles' coordinates (laid out like tiled), boxes, smallest values and
+  // single components are those of SpatialIndex::buildRowTiles; *rowTiles of
+  // the row tiles hold rows, the first of tileOrder (or of 0, 1, ...). Null:
+  // row tile I is column tile I.
+  const int *rowPos, *rowTiles;
+  const float *rowTiled, *rowBoxLow, *rowBoxHigh, *rowMinValue;
+  const int *rowPure;
+
+  // Position of row r of row tile I, -1 when there is none.
+  __device__ __forceinline__ int rowPosition(int I, int r) const {
+    if (rowPos)
+      return rowPos[(size_t)I * kTile + r];
+    const int pos = I * kTile + r;
+    return pos < n ? pos : -1;
+  }
 };
 
-// Index bit of a seed key whose row is settled (indices stay below 2^30).
-constexpr unsigned long long kSettledKey = 1ull << 31;
+// What a block of a pass works on: a row tile against the subtree `root` of
+// the column tiles (root < 0: nothing). A pass over some of the rows may have
+// far fewer row tiles than the GPU has room for, and one block's walk over
+// every column tile would then be the whole pass; so each row tile is shared
+// by 2^splitBits blocks, each taking one subtree at that depth, as many as
+// the launch has blocks for, at most kSplitBlocks in all and with about
+// kSplitTiles column tiles each (fewer would not pay for a block's start).
+// The blocks of a row tile meet in an atomic minimum.
+constexpr int kSplitBlocks = 1184; // four waves of two blocks on 148 SMs
+constexpr int kSplitTiles = 16;
+
+struct BlockWork {
+  int rowTile, root;
+};
+
+__device__ __forceinline__ BlockWork blockWork(const PassParams &p) {
+  int b = blockIdx.x, splitBits = 0, split = 0;
+  if (p.rowPos) {
+    const int tiles = *p.rowTiles;
+    if (tiles <= 0)
+      return {0, -1};
+    while (((tiles << splitBits) * 2LL) <= min((int)gridDim.x, kSplitBlocks) &&
+           (p.numTiles >> splitBits) > kSplitTiles)
+      ++splitBits;
+    split = b / tiles;
+    b %= tiles;
+    if (split >= 1 << splitBits)
+      return {0, -1};
+  }
+  const int I = p.tileOrder ? p.tileOrder[b] : b;
+  int root = p.rootOfTile ? p.rootOfTile[I] : 0;
+  for (int i = 0; i < splitBits; ++i) {
+    const int left = p.nodeLeft[root];
+    if (left < 0) { // a leaf above the split depth: the first block's
+      if (split >> i)
+        root = -1;
+      break;
+    }
+    root = (split >> i) & 1 ? p.nodeRight[root] : left;
+  }
+  return {I, root};
+}
+
+// Slot of entry e of position pos in the k-NN list arrays: tile by tile, each
+// entry's 128 positions contiguous, so that a pass over the positions reads
+// and writes whole lines.
+__host__ __device__ __forceinline__ size_t knnSlot(int pos, int e, int k) {
+  return ((size_t)(pos / kTile) * k + e) * kTile + pos % kTile;
+}
 
 // Lower bound of every distance between the row tile box (shared memory)
 // and a node box, by warp 0 (lanes split the features).

@@ -38,7 +38,8 @@ int pairwiseDistances(const float *A, int nA, const float *B, int nB, int d, con
 
 #define CUHC_INSTANTIATE_CORE(M)                                                                   \
   template int cuhc::coreDistances<M>(cuhc::SpatialIndex &, const M &, int, bool, float *,         \
-                                      cuhc::PassStats *, cudaStream_t, const int *, int *, int *); \
+                                      cuhc::PassStats *, cudaStream_t, const int *,                \
+                                      cuhc::KnnLists *, bool);                                     \
   template bool cuhc::screenable<M>(cuhc::SpatialIndex &, int);                                    \
   template float cuhc::timeKnnSample<M>(cuhc::SpatialIndex &, const M &, int, bool, int, float *,  \
                                         cudaStream_t);                                             \

@@ -59,33 +59,53 @@ void treeFromOrderedMerges(const int *u, const int *v, const float *w, int n, do
 bool mergesFormTree(const std::vector<int> &u, const std::vector<int> &v,
                     const std::vector<float> &w, int n);
 
-// HDBSCAN's k-NN lists (a by-product of the core-distance pass), by
-// position: the positions of each point's k nearest points in ascending
-// distance (itself included) and a flag set when a point outside the list
-// lies at exactly the k-th distance.
+// k-NN lists (a by-product of the k-NN pass), by position: the positions and
+// distances of each point's k nearest points in ascending distance (itself
+// included, +inf past the last when it has fewer) at knnSlot(position, entry,
+// k), and a flag set when a point outside the list lies at exactly the k-th
+// distance.
 struct KnnLists {
-  const int *pos = nullptr;
-  const int *tie = nullptr;
+  int *pos = nullptr;
+  float *val = nullptr;
+  int *tie = nullptr;
   int k = 0;
+  double tilesSearched = 0; // column tiles that the list pass computed
+};
+
+// Device buffers of such lists for n positions.
+struct KnnListBuffers {
+  DeviceBuffer<int> pos, tie;
+  DeviceBuffer<float> val;
+  int allocate(int n, int k, cudaStream_t s) {
+    StatusChain st;
+    CUHC_TRY(st, pos.allocate(paddedToTiles(n) * k, s));
+    CUHC_TRY(st, val.allocate(paddedToTiles(n) * k, s));
+    CUHC_TRY(st, tie.allocate(n, s));
+    return st.code;
+  }
+  KnnLists lists(int k) const { return KnnLists{pos.get(), val.get(), tie.get(), k}; }
 };
 
 // Borůvka over the points of an index (Metric x Weight instantiations in
 // inst_<metric>_mst.cu and inst_<metric>_mreach.cu). Fills edges with the
 // n-1 MST edges (original indices).
-// With knn (mutual reachability, alpha 1), every round first seeds each row
-// with its lightest list edge to another component and settles the rows
-// whose list edge is provably their answer (boruvka.cuh, seedFromKnn).
+// With knn (plain weights, or mutual reachability with alpha 1), every round
+// first seeds each row with its lightest list edge to another component and
+// settles the rows whose list edge is provably their answer (boruvka.cuh,
+// seedRows).
 template <class Metric, class Weight>
 int boruvkaMst(SpatialIndex &index, const Metric &metric, const Weight &weight, bool prune,
                DeviceEdges &edges, PassStats *stats, cudaStream_t stream,
                RadiusLog *radiusLog = nullptr, const KnnLists *knn = nullptr);
 
 // Exact core distances (k-th nearest, the point itself first) by position;
-// with knnPos / knnTie (n x k and n ints) also the k-NN lists (KnnLists).
+// with `lists` also the k-NN lists. `rounds` marks a pass that stands for the
+// first round's nearest search of a single-linkage solve (counted as such by
+// the per-kind timing, and run with the default pipeline shape).
 template <class Metric>
 int coreDistances(SpatialIndex &index, const Metric &metric, int k, bool prune, float *core,
                   PassStats *stats, cudaStream_t stream, const int *coreRank = nullptr,
-                  int *knnPos = nullptr, int *knnTie = nullptr);
+                  KnnLists *lists = nullptr, bool rounds = false);
 
 // The same core distances for any 1 <= k <= n by radix select over chunks of
 // the materialised distance matrix (radix.cuh). Bit-identical to

@@ -71,15 +71,13 @@ struct ColumnMeta {
 template <class Metric, class Weight, bool kKnn>
 __device__ __forceinline__ void refreshThresholds(const PassParams &p, const Metric &m,
                                                   const Weight &w, PassState &sh,
-                                                  const float *lists, int firstRow) {
+                                                  const float *lists, int rowTile) {
   const int tid = threadIdx.x;
   float t = -INFINITY;
   if (tid < kTile) {
-    const int pos = firstRow + tid;
-    // Padding slots and settled rows never search.
-    const bool valid = pos < p.n && p.order[pos] >= 0 &&
-                       !(!kKnn && p.seedKey && (p.seedKey[pos] & kSettledKey) &&
-                         p.seedKey[pos] != kEmptyKey);
+    const int pos = p.rowPosition(rowTile, tid);
+    // Padding slots and inactive rows never search.
+    const bool valid = pos >= 0 && p.order[pos] >= 0 && (kKnn || !p.active || p.active[pos]);
     float thr, filter = -INFINITY;
     if (kKnn) {
       thr = lists[tid * p.k + p.k - 1];
@@ -462,11 +460,21 @@ __global__ void __launch_bounds__(kThreads, 2) passKernel(PassParams p, Metric m
 
   const TileGeom g;
   const int tid = threadIdx.x;
-  const int I = p.tileOrder ? p.tileOrder[blockIdx.x] : (int)blockIdx.x;
+  const BlockWork work = blockWork(p);
+  const int I = work.rowTile;
+  if (work.root < 0)
+    return;
+  if (!kKnn && p.active) {
+    const int pos = tid < kTile ? p.rowPosition(I, tid) : -1;
+    if (!__syncthreads_or(pos >= 0 && p.active[pos]))
+      return; // no row of this tile searches
+  }
   const int firstRow = I * kTile;
   const int leaf = p.leafOfTile[I];
-  const int rowPure = (!kKnn && p.nodePure) ? p.nodePure[leaf] : -1;
-  const float rowMinValue = p.nodeMinValue ? p.nodeMinValue[leaf] : 0.0f;
+  const int rowPure = (!kKnn && p.nodePure) ? (p.rowPos ? p.rowPure[I] : p.nodePure[leaf]) : -1;
+  const float rowMinValue =
+      p.nodeMinValue ? (p.rowPos ? p.rowMinValue[I] : p.nodeMinValue[leaf]) : 0.0f;
+  const float *rowSource = p.rowPos ? p.rowTiled : p.tiled;
   const float slack = 1.0f - boxSlack(p.d);
   const bool useComp = !kKnn && p.component != nullptr;
   const bool useValue = !kKnn && w.value != nullptr;
@@ -476,17 +484,15 @@ __global__ void __launch_bounds__(kThreads, 2) passKernel(PassParams p, Metric m
   float rowVal[8];
 #pragma unroll
   for (int r = 0; r < 8; ++r) {
-    const int pos = firstRow + g.row(r);
-    const bool valid = pos < p.n;
+    const int pos = p.rowPosition(I, g.row(r));
+    const bool valid = pos >= 0;
     rowComp[r] = valid ? (p.component ? p.component[pos] : p.order[pos]) : -2;
     rowVal[r] = valid ? w.load(pos) : 0.0f;
   }
   if (tid < kTile) {
-    const int pos = firstRow + tid;
-    const unsigned long long seed =
-        (!kKnn && p.seedKey && pos < p.n) ? p.seedKey[pos] : kEmptyKey;
-    // A settled row keeps its seed as the answer (written before the pass).
-    sh.rowBest[tid] = (seed & kSettledKey) && seed != kEmptyKey ? kEmptyKey : seed;
+    const int pos = p.rowPosition(I, tid);
+    const bool searches = !kKnn && pos >= 0 && (!p.active || p.active[pos]);
+    sh.rowBest[tid] = searches && p.seedKey ? p.seedKey[pos] : kEmptyKey;
     sh.rowTie[tid] = 0;
   }
   if (kKnn)
@@ -496,26 +502,26 @@ __global__ void __launch_bounds__(kThreads, 2) passKernel(PassParams p, Metric m
         listPos[i] = -1;
     }
   for (int f = tid; f < p.d; f += kThreads) {
-    rowLow[f] = p.nodeLow[(size_t)leaf * p.d + f];
-    rowHigh[f] = p.nodeHigh[(size_t)leaf * p.d + f];
+    rowLow[f] = p.rowPos ? p.rowBoxLow[(size_t)I * p.d + f] : p.nodeLow[(size_t)leaf * p.d + f];
+    rowHigh[f] = p.rowPos ? p.rowBoxHigh[(size_t)I * p.d + f] : p.nodeHigh[(size_t)leaf * p.d + f];
   }
   if (p.numChunks == 1)
-    copyChunk(sA, p.tiled + (size_t)I * tileFloats, KC * kTile);
+    copyChunk(sA, rowSource + (size_t)I * tileFloats, KC * kTile);
   if (tid == 0) {
     mbarrierInit(&sh.bar[0], 1);
     mbarrierInit(&sh.bar[1], 1);
     fenceBarrierInit();
     sh.frontLen = 0;
     sh.overflow = 0;
-    const int root = p.rootOfTile ? p.rootOfTile[I] : 0;
-    const int rootPure = (!kKnn && p.nodePure) ? p.nodePure[root] : -1;
+    const int rootPure = (!kKnn && p.nodePure) ? p.nodePure[work.root] : -1;
     if (!(rowPure >= 0 && rootPure == rowPure)) {
-      sh.frontNode[0] = root;
+      sh.frontNode[0] = work.root;
       sh.frontLen = 1;
     }
   }
-  // Column metadata of the row tile itself, for the self tile.
-  if (tid < kTile) {
+  // Column metadata of the row tile itself, for the self tile (a pass over
+  // some of the rows has none: the walk visits every column tile).
+  if (tid < kTile && !p.rowPos) {
     const int pos = firstRow + tid;
     const bool valid = pos < p.n;
     meta[0].orig[tid] = valid ? p.order[pos] : -1;
@@ -525,7 +531,7 @@ __global__ void __launch_bounds__(kThreads, 2) passKernel(PassParams p, Metric m
       meta[0].value[tid] = valid ? w.load(pos) : 0.0f;
   }
   __syncthreads();
-  refreshThresholds<Metric, Weight, kKnn>(p, m, w, sh, lists, firstRow);
+  refreshThresholds<Metric, Weight, kKnn>(p, m, w, sh, lists, I);
 
   unsigned long long computed = 0;
   bool failed = false;
@@ -550,7 +556,7 @@ __global__ void __launch_bounds__(kThreads, 2) passKernel(PassParams p, Metric m
                                       useComp, useValue,
                                       maskPass && !(rowPure >= 0 && colPure), g, sh.rowBest);
     __syncthreads();
-    refreshThresholds<Metric, Weight, kKnn>(p, m, w, sh, lists, firstRow);
+    refreshThresholds<Metric, Weight, kKnn>(p, m, w, sh, lists, I);
     ++computed;
   };
   // The general path (features in several chunks): synchronous staging.
@@ -565,20 +571,20 @@ __global__ void __launch_bounds__(kThreads, 2) passKernel(PassParams p, Metric m
         meta[0].value[tid] = valid ? w.load(pos) : 0.0f;
     }
     typename Metric::Acc acc[8][8];
-    computeTile<Metric, KC>(p.tiled, p.tiled, p.numChunks, I, J, sA, sB[0], m, acc, g);
+    computeTile<Metric, KC>(rowSource, p.tiled, p.numChunks, I, J, sA, sB[0], m, acc, g);
     if (kKnn)
       knnEpilogue(m, sh, lists, listPos, p.k, acc, firstRow, J * kTile, p.n, meta[0].orig, g);
     else
       nearestEpilogue<Metric, Weight>(m, w, sh, meta[0], acc, rowComp, rowVal, J * kTile, p.n,
                                       useComp, useValue, maskPass, g, sh.rowBest);
     __syncthreads();
-    refreshThresholds<Metric, Weight, kKnn>(p, m, w, sh, lists, firstRow);
+    refreshThresholds<Metric, Weight, kKnn>(p, m, w, sh, lists, I);
     ++computed;
   };
 
   // 1. The row tile against itself (none if all its points share one
   //    component: no edge inside).
-  if (rowPure < 0) {
+  if (rowPure < 0 && !p.rowPos) {
     if (p.numChunks == 1)
       processTile(I, sA, meta[0], false);
     else
@@ -607,7 +613,8 @@ __global__ void __launch_bounds__(kThreads, 2) passKernel(PassParams p, Metric m
   while (!failed) {
     // 2. Candidates of this batch.
     if (tid < 32)
-      collectCandidates(p, m, w, sh, rowLow, rowHigh, I, rowPure, rowMinValue, slack);
+      collectCandidates(p, m, w, sh, rowLow, rowHigh, p.rowPos ? -1 : I, rowPure, rowMinValue,
+                        slack);
     __syncthreads();
     const int len = sh.listLen;
     if (sh.overflow) {
@@ -670,20 +677,23 @@ __global__ void __launch_bounds__(kThreads, 2) passKernel(PassParams p, Metric m
     if (inFlight[b])
       mbarrierWait(&sh.bar[b], phase[b]);
   if (tid < kTile) {
-    const int pos = firstRow + tid;
-    if (pos < p.n) {
+    const int pos = p.rowPosition(I, tid);
+    if (pos >= 0) {
       if (kKnn) {
         const int rank = p.coreRank ? p.coreRank[pos] : p.k;
         p.core[pos] = rank > 0 ? lists[tid * p.k + rank - 1] : 0.0f;
         if (listPos) {
-          for (int e = 0; e < p.k; ++e)
-            p.knnPos[(size_t)pos * p.k + e] = listPos[tid * p.k + e];
+          for (int e = 0; e < p.k; ++e) {
+            p.knnPos[knnSlot(pos, e, p.k)] = listPos[tid * p.k + e];
+            p.knnVal[knnSlot(pos, e, p.k)] = lists[tid * p.k + e];
+          }
           p.knnTie[pos] = sh.rowTie[tid];
         }
-      } else if ((!p.radius || p.radius[pos] >= 0.0f) &&
-                 !(p.seedKey && (p.seedKey[pos] & kSettledKey) &&
-                   p.seedKey[pos] != kEmptyKey)) {
-        p.nearest[pos] = sh.rowBest[tid];
+      } else if ((!p.radius || p.radius[pos] >= 0.0f) && (!p.active || p.active[pos])) {
+        if (p.rowPos)
+          atomicMin(&p.nearest[pos], sh.rowBest[tid]); // other blocks share the row
+        else
+          p.nearest[pos] = sh.rowBest[tid];
       }
     }
   }

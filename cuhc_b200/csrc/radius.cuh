@@ -136,6 +136,8 @@ static __global__ void certifyRows(const unsigned long long *__restrict__ neares
     return;
   const unsigned long long key = nearest[pos];
   const float r = radius[pos];
+  if (r < 0.0f)
+    return; // not proposed: its component sits the round out
   const bool inside = key != kEmptyKey && keyWeight(key) <= r;
   const bool ok = inside || r >= __uint_as_float(compMin[comp[pos]]);
   radius[pos] = ok ? -1.0f : INFINITY;

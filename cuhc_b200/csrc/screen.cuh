@@ -533,11 +533,15 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool consumer = tid < kTile;
   const bool producer = tid == kProducerWarp * 32, mmaThread = tid == kMmaWarp * 32;
-  const int I = p.tileOrder ? p.tileOrder[blockIdx.x] : (int)blockIdx.x;
-  const int firstRow = I * kTile;
+  const BlockWork work = blockWork(p);
+  const int I = work.rowTile;
+  if (work.root < 0)
+    return;
   const int leaf = p.leafOfTile[I];
-  const int rowPure = (!kKnn && p.nodePure) ? p.nodePure[leaf] : -1;
-  const float rowMinValue = p.nodeMinValue ? p.nodeMinValue[leaf] : 0.0f;
+  const bool someRows = !kKnn && p.rowPos != nullptr;
+  const int rowPure = (!kKnn && p.nodePure) ? (someRows ? p.rowPure[I] : p.nodePure[leaf]) : -1;
+  const float rowMinValue =
+      p.nodeMinValue ? (someRows ? p.rowMinValue[I] : p.nodeMinValue[leaf]) : 0.0f;
   const float slack = 1.0f - boxSlack(p.d);
   const bool useComp = !kKnn && p.component != nullptr;
   const bool useValue = !kKnn && w.value != nullptr;
@@ -549,16 +553,18 @@ __global__ void __launch_bounds__(kThreads, 2)
 
   // Consumer row state (thread = row).
   const int myRow = tid & (kTile - 1);
-  const int myPos = firstRow + myRow;
-  const bool myValid = consumer && myPos < p.n && p.order[myPos] >= 0; // not a padding slot
+  const int myPos = p.rowPosition(I, myRow);
+  const bool myValid = consumer && myPos >= 0 && p.order[myPos] >= 0; // not a padding slot
   const int myComp = myValid ? (p.component ? p.component[myPos] : p.order[myPos]) : -2;
   const float myVal = myValid ? w.load(myPos) : 0.0f;
-  // A seed is a real edge of the row; a settled seed is its answer already
-  // (written before the pass): the row neither searches nor writes.
+  // An inactive row's answer was written before the pass: it neither searches
+  // nor writes.
+  const bool mySearch = myValid && (kKnn || !p.active || p.active[myPos]);
+  if (!kKnn && p.active && !__syncthreads_or(mySearch))
+    return; // no row of this tile searches
+  // A seed is a real edge of the row.
   const unsigned long long mySeed =
-      (!kKnn && myValid && p.seedKey) ? p.seedKey[myPos] : kEmptyKey;
-  const bool settled = mySeed != kEmptyKey && (mySeed & kSettledKey) != 0;
-  const bool mySearch = myValid && !settled;
+      (!kKnn && mySearch && p.seedKey) ? p.seedKey[myPos] : kEmptyKey;
   unsigned int *compSlot = (!kKnn && mySearch && p.compBest) ? p.compBest + myComp : nullptr;
 
   if (kKnn)
@@ -567,13 +573,14 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
   for (int f = tid; f < KC; f += kThreads) {
     const bool real = f < p.d;
-    const float lo = real ? p.nodeLow[(size_t)leaf * p.d + f] : 0.0f;
-    const float hi = real ? p.nodeHigh[(size_t)leaf * p.d + f] : 0.0f;
+    const size_t at = (size_t)(someRows ? I : leaf) * p.d + f;
+    const float lo = real ? (someRows ? p.rowBoxLow : p.nodeLow)[at] : 0.0f;
+    const float hi = real ? (someRows ? p.rowBoxHigh : p.nodeHigh)[at] : 0.0f;
     rowLow[f] = lo;
     rowHigh[f] = hi;
     centre[f] = real ? 0.5f * (lo + hi) : 0.0f;
   }
-  copyChunk(sA, p.tiled + (size_t)I * L::rawFloats, KC * kTile);
+  copyChunk(sA, (someRows ? p.rowTiled : p.tiled) + (size_t)I * L::rawFloats, KC * kTile);
   if (warp == 0) {
     tmemAlloc(&ss.tmemBase, 256);
     tmemRelinquish();
@@ -602,10 +609,9 @@ __global__ void __launch_bounds__(kThreads, 2)
     ss.rowSetCount = 0;
     sh.frontLen = 0;
     sh.overflow = 0;
-    const int root = p.rootOfTile ? p.rootOfTile[I] : 0;
-    const int rootPure = (!kKnn && p.nodePure) ? p.nodePure[root] : -1;
+    const int rootPure = (!kKnn && p.nodePure) ? p.nodePure[work.root] : -1;
     if (!(rowPure >= 0 && rootPure == rowPure)) {
-      sh.frontNode[0] = root;
+      sh.frontNode[0] = work.root;
       sh.frontLen = 1;
     }
   }
@@ -675,7 +681,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 
   // Row threshold: sets F (the row's filter bound) and returns the row's
   // threshold for the block maximum (-inf for rows that can gain nothing).
-  unsigned long long rowBest = settled ? kEmptyKey : mySeed;
+  unsigned long long rowBest = mySeed;
   int tie = 0; // k-NN: a point outside the row's list ties its k-th value
   float F = -INFINITY;
   float rowThr = INFINITY; // the row's weight threshold at the last refresh
@@ -722,6 +728,15 @@ __global__ void __launch_bounds__(kThreads, 2)
   __syncthreads();
   if (tid == 0)
     sh.thrTile = fmaxf(fmaxf(ss.warpThr[0], ss.warpThr[1]), fmaxf(ss.warpThr[2], ss.warpThr[3]));
+  // Some rows sit the pass out: the walk's box is that of the rows that
+  // search (the centre, already used, may stay the whole tile's).
+  if (!kKnn && p.active)
+    for (int f = tid; f < p.d; f += kThreads) {
+      rowLow[f] = fminf(fminf(groupLow[f], groupLow[KC + f]),
+                        fminf(groupLow[2 * KC + f], groupLow[3 * KC + f]));
+      rowHigh[f] = fmaxf(fmaxf(groupHigh[f], groupHigh[KC + f]),
+                         fmaxf(groupHigh[2 * KC + f], groupHigh[3 * KC + f]));
+    }
   __syncthreads();
 
   const uint32_t idesc = umma_idesc_tf32(128, 128);
@@ -744,7 +759,9 @@ __global__ void __launch_bounds__(kThreads, 2)
   int lastCommit = -1;
   unsigned long long prefiltered = 0; // candidate tiles no row needed (per thread)
   unsigned long long computed = 0;
-  bool selfPending = kKnn || rowPure < 0;
+  // A pass over some of the rows has no self tile: the walk visits every
+  // column tile.
+  bool selfPending = kKnn || (rowPure < 0 && !someRows);
   bool overflow = false;
   bool dirty = false;                          // consumer: row filter may have tightened
   unsigned long long rechecks = 0, slowRows = 0; // consumer counters
@@ -801,7 +818,8 @@ __global__ void __launch_bounds__(kThreads, 2)
   int batch = 0;
   while (true) {
     if (warp == 0)
-      collectCandidates(p, m, w, sh, rowLow, rowHigh, I, rowPure, rowMinValue, slack);
+      collectCandidates(p, m, w, sh, rowLow, rowHigh, someRows ? -1 : I, rowPure, rowMinValue,
+                        slack);
     __syncthreads();
     const int len = sh.listLen;
     if (sh.overflow) {
@@ -1198,17 +1216,23 @@ __global__ void __launch_bounds__(kThreads, 2)
       mbarrierWait(&ss.rawFull[o % S], (o / S) & 1);
   if (mmaThread && ss.failed && lastCommit >= 0)
     mbarrierWait(&ss.mmaFull[lastCommit & 1], (lastCommit >> 1) & 1);
-  if (consumer && myPos < p.n) {
+  if (consumer && myPos >= 0) {
     if (kKnn) {
       const int rank = myValid ? (p.coreRank ? p.coreRank[myPos] : p.k) : 0;
       p.core[myPos] = rank > 0 ? listKeyValue(lists[myRow * p.k + rank - 1]) : 0.0f;
       if (p.knnPos) {
-        for (int e = 0; e < p.k; ++e)
-          p.knnPos[(size_t)myPos * p.k + e] = (int)(uint32_t)lists[myRow * p.k + e];
+        for (int e = 0; e < p.k; ++e) {
+          const unsigned long long key = lists[myRow * p.k + e];
+          p.knnPos[knnSlot(myPos, e, p.k)] = (int)(uint32_t)key;
+          p.knnVal[knnSlot(myPos, e, p.k)] = listKeyValue(key);
+        }
         p.knnTie[myPos] = tie;
       }
-    } else if ((!p.radius || p.radius[myPos] >= 0.0f) && !settled) {
-      p.nearest[myPos] = rowBest;
+    } else if ((!p.radius || p.radius[myPos] >= 0.0f) && (mySearch || !p.active)) {
+      if (!someRows)
+        p.nearest[myPos] = rowBest;
+      else if (rowBest < mySeed)
+        atomicMin(&p.nearest[myPos], rowBest); // other blocks share the row
     }
   }
   if (consumer && p.screenStats) {

@@ -3,9 +3,12 @@
 #include "spatial.cuh"
 
 #include <algorithm>
+#include <climits>
 #include <cstring>
 #include <vector>
 #include <cub/device/device_radix_sort.cuh>
+#include <cub/device/device_select.cuh>
+#include <cub/iterator/counting_input_iterator.cuh>
 
 namespace cuhc {
 
@@ -620,7 +623,7 @@ __global__ void tileKeysFromWork(const unsigned int *__restrict__ work, int numT
 
 } // namespace
 
-int SpatialIndex::orderTiles(bool fromBoxes, bool impureFirst) {
+int SpatialIndex::allocateTileOrder() {
   StatusChain st;
   if (!tileOrder.get()) {
     CUHC_TRY(st, tileWork.allocate(numTiles, stream));
@@ -633,9 +636,15 @@ int SpatialIndex::orderTiles(bool fromBoxes, bool impureFirst) {
                      tileOrder.get(), numTiles, 0, 32, stream));
     CUHC_TRY(st, tileSortTemp.allocate(std::max<size_t>(tileSortBytes, 1), stream));
     CUHC_TRY(st, cudaMemsetAsync(tileWork.get(), 0, numTiles * sizeof(unsigned int), stream));
-    if (!st.ok())
-      return st.code;
   }
+  return st.code;
+}
+
+int SpatialIndex::orderTiles(bool fromBoxes, bool impureFirst) {
+  StatusChain st;
+  CUHC_TRY(st, allocateTileOrder());
+  if (!st.ok())
+    return st.code;
   if (fromBoxes)
     tileKeysFromBoxes<<<blocksFor(numTiles, 256), 256, 0, stream>>>(
         nodeLow.get(), nodeHigh.get(), leafOfTile.get(), d, numTiles, tileKeys.get(),
@@ -646,9 +655,220 @@ int SpatialIndex::orderTiles(bool fromBoxes, bool impureFirst) {
         tileKeys.get(), tileIota.get());
   noteLaunch();
   CUHC_TRY(st, cudaGetLastError());
-  CUHC_TRY(st, cub::DeviceRadixSort::SortPairsDescending(
-                   tileSortTemp.get(), tileSortBytes, tileKeys.get(), tileKeysSorted.get(),
-                   tileIota.get(), tileOrder.get(), numTiles, 0, 32, stream));
+  CUHC_TRY(st, sortTileKeys());
+  return st.code;
+}
+
+int SpatialIndex::sortTileKeys() {
+  return (int)cub::DeviceRadixSort::SortPairsDescending(
+      tileSortTemp.get(), tileSortBytes, tileKeys.get(), tileKeysSorted.get(), tileIota.get(),
+      tileOrder.get(), numTiles, 0, 32, stream);
+}
+
+double SpatialIndex::fullTilePairs() const {
+  double pairs = 0.0;
+  for (int i = 0; i < numInstances; ++i) {
+    const double tiles =
+        (i + 1 < numInstances ? instanceFirstTile[i + 1] : numTiles) - instanceFirstTile[i];
+    pairs += tiles * tiles;
+  }
+  return pairs;
+}
+
+bool SpatialIndex::orderMatters() const {
+  static const int sms = [] {
+    int device = 0, count = 0;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device);
+    return count;
+  }();
+  return numTiles > 2 * sms;
+}
+
+namespace {
+
+// One block per instance: packs its flagged positions, in order, into its own
+// row tiles and marks the remaining slots empty. first[i] is the instance's
+// first tile (first[gridDim.x]: all tiles); a null `first` is one instance.
+// A chunk of 1024 positions per step: a ballot per warp, a scan of the 32
+// warp counts.
+__global__ void __launch_bounds__(1024)
+    selectInstanceRows(const unsigned char *__restrict__ flag, const int *__restrict__ first,
+                       int numTiles, int n, int *__restrict__ rowPos) {
+  __shared__ int warpCount[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int begin = first ? first[blockIdx.x] * kTile : 0;
+  const int end = first ? first[blockIdx.x + 1] * kTile : numTiles * kTile;
+  int filled = begin;
+  for (int base = begin; base < end; base += 1024) {
+    const int pos = base + threadIdx.x;
+    const bool take = pos < end && pos < n && flag[pos] != 0;
+    const unsigned bits = __ballot_sync(0xffffffffu, take);
+    if (lane == 0)
+      warpCount[warp] = __popc(bits);
+    __syncthreads();
+    int before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < 32; ++w) {
+      before += w < warp ? warpCount[w] : 0;
+      all += warpCount[w];
+    }
+    if (take)
+      rowPos[filled + before + __popc(bits & ((1u << lane) - 1))] = pos;
+    filled += all;
+    __syncthreads();
+  }
+  for (int slot = filled + threadIdx.x; slot < end; slot += 1024)
+    rowPos[slot] = -1;
+}
+
+// Marks the slots past the selected rows empty.
+__global__ void clearUnselected(const int *__restrict__ count, int slots,
+                                int *__restrict__ rowPos) {
+  const int slot = blockIdx.x * blockDim.x + threadIdx.x;
+  if (slot < slots && slot >= *count)
+    rowPos[slot] = -1;
+}
+
+// One block of 128 threads per row tile (thread = row): gathers the rows'
+// coordinates into the tiled layout and reduces their box, smallest value and
+// single component (-1: several). key <- the largest tileWork of the rows' own
+// tiles (0 for an empty row tile).
+__global__ void __launch_bounds__(kTile)
+    buildRowTiles(const float *__restrict__ tiled, const int *__restrict__ rowPos, int d, int kc,
+                  int numChunks, const int *__restrict__ component,
+                  const float *__restrict__ values, const unsigned int *__restrict__ work,
+                  float *__restrict__ rowTiled, float *__restrict__ boxLow,
+                  float *__restrict__ boxHigh, float *__restrict__ minValue,
+                  int *__restrict__ pure, int *__restrict__ filledTiles,
+                  unsigned int *__restrict__ key, int *__restrict__ iota) {
+  __shared__ float sLow[4], sHigh[4], sMin[4];
+  __shared__ int sMax[4], sCompLow[4], sCompHigh[4];
+  const int I = blockIdx.x, r = threadIdx.x, lane = r & 31, warp = r >> 5;
+  const int pos = rowPos[(size_t)I * kTile + r];
+  if (r == 0 && key)
+    iota[I] = I;
+  if (!__syncthreads_or(pos >= 0)) {
+    if (r == 0 && key)
+      key[I] = 0;
+    return;
+  }
+  if (r == 0)
+    atomicAdd(filledTiles, 1);
+  const size_t tileFloats = (size_t)numChunks * kc * kTile;
+  const float *src = pos >= 0 ? tiled + (size_t)(pos / kTile) * tileFloats + pos % kTile : nullptr;
+  float *dst = rowTiled + (size_t)I * tileFloats + r;
+  for (int f = 0; f < numChunks * kc; ++f) {
+    const float x = src ? src[(size_t)f * kTile] : 0.0f;
+    dst[(size_t)f * kTile] = x;
+    if (f >= d)
+      continue;
+    float lo = src ? x : INFINITY, hi = src ? x : -INFINITY;
+    for (int off = 16; off > 0; off /= 2) {
+      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, off));
+      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, off));
+    }
+    if (lane == 0) {
+      sLow[warp] = lo;
+      sHigh[warp] = hi;
+    }
+    __syncthreads();
+    if (r == 0) {
+      boxLow[(size_t)I * d + f] = fminf(fminf(sLow[0], sLow[1]), fminf(sLow[2], sLow[3]));
+      boxHigh[(size_t)I * d + f] = fmaxf(fmaxf(sHigh[0], sHigh[1]), fmaxf(sHigh[2], sHigh[3]));
+    }
+    __syncthreads();
+  }
+  float mn = pos >= 0 && values ? values[pos] : INFINITY;
+  const int c = pos >= 0 && component ? component[pos] : 0;
+  int cLow = pos >= 0 ? c : INT_MAX, cHigh = pos >= 0 ? c : -1;
+  int heavy = pos >= 0 && key ? (int)min(work[pos / kTile], 0x7fffffffu) : 0;
+  for (int off = 16; off > 0; off /= 2) {
+    mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, off));
+    cLow = min(cLow, __shfl_xor_sync(0xffffffffu, cLow, off));
+    cHigh = max(cHigh, __shfl_xor_sync(0xffffffffu, cHigh, off));
+    heavy = max(heavy, __shfl_xor_sync(0xffffffffu, heavy, off));
+  }
+  if (lane == 0) {
+    sMin[warp] = mn;
+    sCompLow[warp] = cLow;
+    sCompHigh[warp] = cHigh;
+    sMax[warp] = heavy;
+  }
+  __syncthreads();
+  if (r == 0) {
+    const float m4 = fminf(fminf(sMin[0], sMin[1]), fminf(sMin[2], sMin[3]));
+    minValue[I] = values ? m4 : 0.0f;
+    const int low = min(min(sCompLow[0], sCompLow[1]), min(sCompLow[2], sCompLow[3]));
+    const int high = max(max(sCompHigh[0], sCompHigh[1]), max(sCompHigh[2], sCompHigh[3]));
+    pure[I] = component && low == high ? low : -1;
+    // Row tiles of several components first, each group heaviest first (as
+    // orderTiles: boundary rows tighten the components' bests early).
+    if (key)
+      key[I] = ((unsigned int)max(max(sMax[0], sMax[1]), max(sMax[2], sMax[3])) >> 1) + 1 |
+               (low != high ? 0x80000000u : 0u);
+  }
+}
+
+} // namespace
+
+int SpatialIndex::selectRows(const unsigned char *flag, const int *component,
+                             const float *values, bool *ordered) {
+  StatusChain st;
+  const bool order = numInstances > 1 || orderMatters();
+  *ordered = order;
+  if (order)
+    CUHC_TRY(st, allocateTileOrder());
+  const int slots = numTiles * kTile;
+  // One block walks an instance 1024 positions a step (about a microsecond
+  // each); a larger single instance goes through a device-wide select.
+  const bool perInstance = numInstances > 1 || n <= 16384;
+  if (!rowPos.get()) {
+    CUHC_TRY(st, rowPos.allocate(slots, stream));
+    CUHC_TRY(st, rowPure.allocate(numTiles, stream));
+    CUHC_TRY(st, rowTiled.allocate((size_t)numTiles * tileFloats(), stream));
+    CUHC_TRY(st, rowBoxLow.allocate((size_t)numTiles * d, stream));
+    CUHC_TRY(st, rowBoxHigh.allocate((size_t)numTiles * d, stream));
+    CUHC_TRY(st, rowMinValue.allocate(numTiles, stream));
+    CUHC_TRY(st, rowCount.allocate(1, stream));
+    CUHC_TRY(st, rowTiles.allocate(1, stream));
+    if (!perInstance) {
+      CUHC_TRY(st, cub::DeviceSelect::Flagged(nullptr, selectBytes,
+                                              cub::CountingInputIterator<int>(0), flag,
+                                              rowPos.get(), rowCount.get(), n, stream));
+      CUHC_TRY(st, selectTemp.allocate(std::max<size_t>(selectBytes, 1), stream));
+    }
+    if (numInstances > 1) {
+      std::vector<int> first(instanceFirstTile);
+      first.push_back(numTiles);
+      CUHC_TRY(st, instanceTile.allocate(first.size(), stream));
+      CUHC_TRY(st, cudaMemcpyAsync(instanceTile.get(), first.data(), first.size() * sizeof(int),
+                                   cudaMemcpyHostToDevice, stream));
+      CUHC_TRY(st, cudaStreamSynchronize(stream));
+    }
+  }
+  if (!st.ok())
+    return st.code;
+  if (perInstance) {
+    selectInstanceRows<<<numInstances, 1024, 0, stream>>>(
+        flag, numInstances > 1 ? instanceTile.get() : nullptr, numTiles, n, rowPos.get());
+  } else {
+    CUHC_TRY(st, cub::DeviceSelect::Flagged(selectTemp.get(), selectBytes,
+                                            cub::CountingInputIterator<int>(0), flag,
+                                            rowPos.get(), rowCount.get(), n, stream));
+    clearUnselected<<<blocksFor(slots, 256), 256, 0, stream>>>(rowCount.get(), slots,
+                                                               rowPos.get());
+  }
+  noteLaunch();
+  CUHC_TRY(st, cudaMemsetAsync(rowTiles.get(), 0, sizeof(int), stream));
+  buildRowTiles<<<numTiles, kTile, 0, stream>>>(
+      tiled.get(), rowPos.get(), d, kc, numChunks, component, values, tileWork.get(),
+      rowTiled.get(), rowBoxLow.get(), rowBoxHigh.get(), rowMinValue.get(), rowPure.get(),
+      rowTiles.get(), order ? tileKeys.get() : nullptr, order ? tileIota.get() : nullptr);
+  noteLaunch();
+  CUHC_TRY(st, cudaGetLastError());
+  if (order)
+    CUHC_TRY(st, sortTileKeys());
   return st.code;
 }
 

@@ -67,6 +67,15 @@ struct SpatialIndex {
   DeviceBuffer<unsigned char> tileSortTemp;
   size_t tileSortBytes = 0;
   bool tileWorkValid = false;            // a pass has recorded tileWork
+  // A pass over some of the rows (selectRows, buildRowTiles): the rows'
+  // positions in row tiles of 128, and per row tile the coordinates (laid
+  // out like tiled), box, smallest value and single component.
+  DeviceBuffer<int> rowPos, rowPure, rowTiles; // rowTiles: row tiles that hold rows
+  DeviceBuffer<float> rowTiled, rowBoxLow, rowBoxHigh, rowMinValue;
+  DeviceBuffer<int> rowCount;            // selected rows (one instance)
+  DeviceBuffer<unsigned char> selectTemp;
+  DeviceBuffer<int> instanceTile;        // first tile per instance, then numTiles (batches)
+  size_t selectBytes = 0;
 
   size_t tileFloats() const { return (size_t)numChunks * kc * kTile; }
 
@@ -102,6 +111,23 @@ struct SpatialIndex {
   // impureFirst: row tiles whose points span several components (nodePure
   // of the round) go before the others, each group heaviest first.
   int orderTiles(bool fromBoxes, bool impureFirst = false);
+  // Whether a pass's launch order can matter: at most two blocks of a pass
+  // share an SM, so with no more row tiles than that all start at once.
+  bool orderMatters() const;
+  // Tile pairs of a pass without pruning (a batch: inside its instances).
+  double fullTilePairs() const;
+  // rowPos <- the positions with flag[position] != 0, in position order and
+  // packed into row tiles; a batch packs each instance into its own tiles,
+  // so that a row tile never spans instances. Then the row tiles' data
+  // (component and values by position, null: none), their number and, for a
+  // batch or where it matters, tileOrder: heaviest first by the work of the
+  // rows' own tiles in the last full pass, row tiles without rows last.
+  // *ordered tells whether it is in use. Enqueued on the index stream with no
+  // host work (buffers are allocated on first use).
+  int selectRows(const unsigned char *flag, const int *componentByPosition,
+                 const float *valuesByPosition, bool *ordered);
+  int allocateTileOrder();
+  int sortTileKeys();
 };
 
 } // namespace cuhc
