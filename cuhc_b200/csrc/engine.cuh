@@ -162,7 +162,8 @@ struct PassParams {
   const int *coreRank;    // knn-mode rank per position, 0 = core 0 (null: k for all)
   // Nearest mode: per-position cap on the row threshold (a proposed radius);
   // a negative value marks a row that is already settled: it neither
-  // searches nor writes. Null: no cap.
+  // searches nor writes. Knn mode with a weight: partners heavier than this
+  // need not be found. Null: no cap.
   const float *radius;
   // Block b takes row tile tileOrder[b] (null: b), so that the heaviest row
   // tiles start first; tileWork[I] receives the column tiles row tile I
@@ -175,6 +176,11 @@ struct PassParams {
   int *knnPos;
   float *knnVal;
   int *knnTie;
+  // Knn mode with a weight (the row itself left out): each block's lists as
+  // keys (weight bits << 32 | original index), the k lightest in that order,
+  // [block][entry][row]; entries past the last hold kEmptyListKey. A row
+  // tile's blocks hold one part each.
+  unsigned long long *knnParts;
   // Nearest mode: per position an initial best key (a real edge of the row,
   // kEmptyKey: none; null: no seeds), and whether the row searches (null: all
   // do); a row that does not keeps what `nearest` holds.
@@ -220,15 +226,30 @@ struct BlockWork {
   int rowTile, root;
 };
 
+// A list entry of the k-NN modes as a key: value bits << 32 | position (or
+// original index), so that keys order by value (values are clamped at +0, so
+// their bits order like the floats), then by index. An empty entry holds +inf.
+constexpr unsigned long long kEmptyListKey = 0x7f800000ffffffffull;
+
+__device__ __forceinline__ float listKeyValue(unsigned long long key) {
+  return __uint_as_float((uint32_t)(key >> 32));
+}
+
+__device__ __forceinline__ int splitBitsFor(int tiles, int numBlocks, int numTiles) {
+  int bits = 0;
+  while (((tiles << bits) * 2LL) <= min(numBlocks, kSplitBlocks) &&
+         (numTiles >> bits) > kSplitTiles)
+    ++bits;
+  return bits;
+}
+
 __device__ __forceinline__ BlockWork blockWork(const PassParams &p) {
   int b = blockIdx.x, splitBits = 0, split = 0;
   if (p.rowPos) {
     const int tiles = *p.rowTiles;
     if (tiles <= 0)
       return {0, -1};
-    while (((tiles << splitBits) * 2LL) <= min((int)gridDim.x, kSplitBlocks) &&
-           (p.numTiles >> splitBits) > kSplitTiles)
-      ++splitBits;
+    splitBits = splitBitsFor(tiles, gridDim.x, p.numTiles);
     split = b / tiles;
     b %= tiles;
     if (split >= 1 << splitBits)

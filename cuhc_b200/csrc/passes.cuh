@@ -30,6 +30,8 @@
 //   5. repeat from 2 until the frontier is empty.
 #pragma once
 
+#include <type_traits>
+
 #include "asyncload.cuh"
 #include "engine.cuh"
 #include "profiling.cuh"
@@ -81,8 +83,10 @@ __device__ __forceinline__ void refreshThresholds(const PassParams &p, const Met
     float thr, filter = -INFINITY;
     if (kKnn) {
       thr = lists[tid * p.k + p.k - 1];
+      if (valid && !std::is_same<Weight, PlainWeight>::value && p.radius)
+        thr = fminf(thr, p.radius[pos]);
       if (valid)
-        filter = m.filterBound(thr);
+        filter = m.filterBound(w.distBound(thr, w.load(pos)));
     } else {
       const unsigned long long key = sh.rowBest[tid];
       thr = key == kEmptyKey ? INFINITY : keyWeight(key);
@@ -259,31 +263,52 @@ __device__ __forceinline__ bool knnOffer(float *list, int *pos, int k, float v, 
   return false;
 }
 
-template <class Metric>
-__device__ __forceinline__ void knnEpilogue(const Metric &m, PassState &sh, float *lists,
-                                            int *listPos, int k,
-                                            typename Metric::Acc (&acc)[8][8], int firstRow,
-                                            int firstCol, int n, const int *colOrig,
-                                            const TileGeom &g) {
+// Offers weight v of original index j to a row's list, kept in (weight, index)
+// order, so that the first entry is the row's answer whatever the ties.
+__device__ __forceinline__ void offerByIndex(float *list, int *index, int k, float v, int j) {
+  if (!(v < INFINITY)) // NaN too
+    return;
+  v = v > 0.0f ? v : 0.0f;
+  if (v > list[k - 1] || (v == list[k - 1] && j > index[k - 1]))
+    return;
+  int i = k - 1;
+  for (; i > 0 && (list[i - 1] > v || (list[i - 1] == v && index[i - 1] > j)); --i) {
+    list[i] = list[i - 1];
+    index[i] = index[i - 1];
+  }
+  list[i] = v;
+  index[i] = j;
+}
+
+template <class Metric, class Weight>
+__device__ __forceinline__ void knnEpilogue(const PassParams &p, const Metric &m, const Weight &w,
+                                            PassState &sh, float *lists, int *listPos, int k,
+                                            typename Metric::Acc (&acc)[8][8], int rowTile,
+                                            const float (&rowVal)[8], int firstCol, int n,
+                                            const ColumnMeta &cm, const TileGeom &g) {
+  // By weight (the row itself left out) or by distance (it counts as 0).
+  constexpr bool kWeighted = !std::is_same<Weight, PlainWeight>::value;
+  const int *colOrig = cm.orig;
   const int lane = threadIdx.x & 31;
   const unsigned groupMask = (lane < 16) ? 0x0000ffffu : 0xffff0000u;
 #pragma unroll
   for (int r = 0; r < 8; ++r) {
     const int rowInTile = g.row(r);
-    const int rowPos = firstRow + rowInTile;
+    const int rowPos = p.rowPosition(rowTile, rowInTile);
     float *list = lists + rowInTile * k;
     const float F = sh.rowFilter[rowInTile];
     float mn = INFINITY;
 #pragma unroll
     for (int c = 0; c < 8; ++c)
       mn = fminf(mn, m.filter(acc[r][c]));
-    if (!__any_sync(0xffffffffu, rowPos < n && mn <= F))
+    if (!__any_sync(0xffffffffu, rowPos >= 0 && mn <= F))
       continue; // no pair of this row group can enter a list
     unsigned pending = 0;
-    if (rowPos < n) {
+    if (rowPos >= 0) {
 #pragma unroll
       for (int c = 0; c < 8; ++c)
-        if (firstCol + g.col(c) < n && colOrig[g.col(c)] >= 0 && m.filter(acc[r][c]) <= F)
+        if (firstCol + g.col(c) < n && colOrig[g.col(c)] >= 0 && m.filter(acc[r][c]) <= F &&
+            !(kWeighted && firstCol + g.col(c) == rowPos))
           pending |= 1u << c;
     }
     while (true) {
@@ -301,9 +326,15 @@ __device__ __forceinline__ void knnEpilogue(const Metric &m, PassState &sh, floa
             a = acc[r][cc];
         const int colPos = firstCol + g.col(c);
         // The point itself counts as distance 0 (hdbscan.cuh:205-212).
-        const float v = colPos == rowPos ? 0.0f : fmaxf(m.finalize(a), 0.0f);
-        knnOffer(list, listPos ? listPos + rowInTile * k : nullptr, k, v, colPos,
-                 sh.rowTie[rowInTile]);
+        const float v = kWeighted
+                            ? w.weight(m.finalize(a), rowVal[r], cm.value[g.col(c)])
+                        : colPos == rowPos ? 0.0f
+                                           : fmaxf(m.finalize(a), 0.0f);
+        if (kWeighted)
+          offerByIndex(list, listPos + rowInTile * k, k, v, colOrig[g.col(c)]);
+        else
+          knnOffer(list, listPos ? listPos + rowInTile * k : nullptr, k, v, colPos,
+                   sh.rowTie[rowInTile]);
       }
       __syncwarp();
     }
@@ -456,7 +487,9 @@ __global__ void __launch_bounds__(kThreads, 2) passKernel(PassParams p, Metric m
   float *rowLow = (float *)(metaBase + 6 * kTile);
   float *rowHigh = rowLow + p.d;
   float *lists = rowHigh + p.d;
-  int *listPos = (kKnn && p.knnPos) ? reinterpret_cast<int *>(lists + kTile * p.k) : nullptr;
+  constexpr bool kWeighted = kKnn && !std::is_same<Weight, PlainWeight>::value;
+  int *listPos = (kKnn && (p.knnPos || kWeighted)) ? reinterpret_cast<int *>(lists + kTile * p.k)
+                                                   : nullptr;
 
   const TileGeom g;
   const int tid = threadIdx.x;
@@ -477,7 +510,7 @@ __global__ void __launch_bounds__(kThreads, 2) passKernel(PassParams p, Metric m
   const float *rowSource = p.rowPos ? p.rowTiled : p.tiled;
   const float slack = 1.0f - boxSlack(p.d);
   const bool useComp = !kKnn && p.component != nullptr;
-  const bool useValue = !kKnn && w.value != nullptr;
+  const bool useValue = (!kKnn || kWeighted) && w.value != nullptr;
   const size_t tileFloats = (size_t)p.numChunks * KC * kTile;
 
   int rowComp[8];
@@ -550,7 +583,7 @@ __global__ void __launch_bounds__(kThreads, 2) passKernel(PassParams p, Metric m
         acc[r][c] = m.init();
     accumulateChunk<Metric, KC>(sA, bTile, m, acc, g);
     if (kKnn)
-      knnEpilogue(m, sh, lists, listPos, p.k, acc, firstRow, J * kTile, p.n, cm.orig, g);
+      knnEpilogue(p, m, w, sh, lists, listPos, p.k, acc, I, rowVal, J * kTile, p.n, cm, g);
     else
       nearestEpilogue<Metric, Weight>(m, w, sh, cm, acc, rowComp, rowVal, J * kTile, p.n,
                                       useComp, useValue,
@@ -573,7 +606,7 @@ __global__ void __launch_bounds__(kThreads, 2) passKernel(PassParams p, Metric m
     typename Metric::Acc acc[8][8];
     computeTile<Metric, KC>(rowSource, p.tiled, p.numChunks, I, J, sA, sB[0], m, acc, g);
     if (kKnn)
-      knnEpilogue(m, sh, lists, listPos, p.k, acc, firstRow, J * kTile, p.n, meta[0].orig, g);
+      knnEpilogue(p, m, w, sh, lists, listPos, p.k, acc, I, rowVal, J * kTile, p.n, meta[0], g);
     else
       nearestEpilogue<Metric, Weight>(m, w, sh, meta[0], acc, rowComp, rowVal, J * kTile, p.n,
                                       useComp, useValue, maskPass, g, sh.rowBest);
@@ -676,7 +709,15 @@ __global__ void __launch_bounds__(kThreads, 2) passKernel(PassParams p, Metric m
   for (int b = 0; b < 2; ++b)
     if (inFlight[b])
       mbarrierWait(&sh.bar[b], phase[b]);
-  if (tid < kTile) {
+  if (kWeighted && tid < kTile)
+    for (int e = 0; e < p.k; ++e) {
+      const float v = lists[tid * p.k + e];
+      p.knnParts[((size_t)blockIdx.x * p.k + e) * kTile + tid] =
+          v < INFINITY ? ((unsigned long long)floatBits(fmaxf(v, 0.0f)) << 32) |
+                             (uint32_t)listPos[tid * p.k + e]
+                       : kEmptyListKey;
+    }
+  if (tid < kTile && !kWeighted) {
     const int pos = p.rowPosition(I, tid);
     if (pos >= 0) {
       if (kKnn) {
@@ -711,7 +752,8 @@ __global__ void __launch_bounds__(kThreads, 2) passKernel(PassParams p, Metric m
 template <class Metric, class Weight, bool kKnn>
 int launchPass(const PassParams &p, const Metric &m, const Weight &w, int kc,
                cudaStream_t stream) {
-  const size_t listEntries = kKnn ? (size_t)kTile * p.k * (p.knnPos ? 2 : 1) : 0;
+  constexpr bool kWeighted = kKnn && !std::is_same<Weight, PlainWeight>::value;
+  const size_t listEntries = kKnn ? (size_t)kTile * p.k * (p.knnPos || kWeighted ? 2 : 1) : 0;
   const size_t dynBytes = (size_t)3 * kc * kTile * sizeof(float) + 6 * kTile * sizeof(int) +
                           (2 * (size_t)p.d + listEntries) * sizeof(float);
   // Bulk copies need 16-byte aligned sources (pool allocations are 256-byte

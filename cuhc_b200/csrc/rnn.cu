@@ -14,10 +14,26 @@
 // from the lower-representative cluster. Without pruning the reference keeps
 // its slots in representative order (compaction preserves it), so this is
 // the reference's arithmetic bit for bit, whatever the physical order.
+//
+// A round changes few clusters, so nearest neighbours are kept across rounds.
+// Every cluster i holds a list of its kListK lightest partners (as of its last
+// search) and a lower bound b_i of its exact weight W(i, c) to every cluster c
+// that is not in the list. Ward's weight is reducible: for a merged pair (a, b)
+// of reciprocal nearest neighbours and a third cluster, W(i, a u b) >=
+// min(W(i, a), W(i, b)). So when clusters outside the list merge, b_i stays a
+// bound; when a list member merges, the merged cluster takes its place with its
+// new exact weight; and when i itself merges with j, the union of their lists
+// and the smaller bound describe the merged row. Rounding costs the bound a
+// little each round (updateLists). A row whose best list weight is below its
+// bound has its answer: every other cluster is heavier. Only the other rows
+// (15 % in the middle rounds of 200,000 x 32) search again, packed into row
+// tiles of their own, capped near the heaviest partner they still know. Ward of
+// 200,000 x 32: 690 -> 172 ms.
 #include "profiling.cuh"
 #include "rnn.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 #include <vector>
@@ -98,8 +114,11 @@ __global__ void rnnMerge(const float *__restrict__ cent, const int *__restrict__
                          const int *__restrict__ newIndex, int m, int d, float *__restrict__ nextCent,
                          int *__restrict__ nextSize, float *__restrict__ nextSizeF,
                          int *__restrict__ nextRep, int *__restrict__ slotOfRep,
-                         int *__restrict__ mergeU, int *__restrict__ mergeV,
-                         float *__restrict__ mergeH, int *__restrict__ mergeCount, int capacity) {
+                         unsigned char *__restrict__ nextChanged,
+                         float *__restrict__ nextMergeWeight,
+                         const unsigned long long *__restrict__ nearest, int *__restrict__ mergeU,
+                         int *__restrict__ mergeV, float *__restrict__ mergeH,
+                         int *__restrict__ mergeCount, int capacity) {
   const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (e >= (long long)m * d)
     return;
@@ -122,7 +141,10 @@ __global__ void rnnMerge(const float *__restrict__ cent, const int *__restrict__
     nextSizeF[to] = (float)merged;
     nextRep[to] = rep[i];
     slotOfRep[rep[i]] = to;
+    nextChanged[to] = j >= 0;
     if (j >= 0) {
+      slotOfRep[rep[j]] = to; // where the lists that name j find it now
+      nextMergeWeight[to] = keyWeight(nearest[i]);
       const float *a = cent + (size_t)i * d, *b = cent + (size_t)j * d;
       float squared = 0.0f;
       for (int k = 0; k < d; ++k) {
@@ -137,6 +159,221 @@ __global__ void rnnMerge(const float *__restrict__ cent, const int *__restrict__
       }
     }
   }
+}
+
+// Entries of a cluster's list. Longer lists last more rounds but widen the
+// search radius; odd, so that rows spread over the shared-memory banks. Whole
+// calls of 200,000 x 32 in ms for 5 / 7 / 9 / 13 entries: 281 / 186 / 190 /
+// 206 (5 measured before the size term of screen.cuh got its updates).
+constexpr int kListK = 7;
+
+// With this many clusters or fewer every round searches all of them: the full
+// pass is then cheaper than the launches that would spare part of it (200,000 x
+// 32: a round at 4,000 clusters takes 0.2 ms with lists and 0.5 without, below
+// 800 about 0.15 either way; 3,916 x 8 in all, mostly such rounds: 10.1 ms with
+// lists throughout, 9.35 without).
+constexpr int kSearchAllBelow = 1024;
+
+// The lists of all clusters, entry-major ([entry][slot], `stride` slots):
+// partners by representative and their exact weights, lightest first by (weight,
+// representative), -1 / +inf past the last; the square root of the bound b.
+struct WardLists {
+  int *rep;
+  float *weight;
+  float *rootBound;
+  size_t stride;
+};
+
+// Relative and absolute rounding of one round, for the bounds. eps bounds the
+// relative error of a computed weight against the exact one (the squared
+// distance's chain, the size products and the fast division: (d + 12) units of
+// rounding, taken 1.5 times over). delta bounds the distance between a stored
+// merged centroid and the exact mean: per feature at most 3.01 u |c_j - c_i| +
+// u |c|, with the data's extent and largest magnitude.
+struct WardRounding {
+  float eps, delta;
+};
+
+// The weights' relative error model needs normal arithmetic: rows with lighter
+// weights search every round, and no bound exceeds kBoundMax (a list may be
+// short because the weights of the other clusters overflow).
+constexpr float kWeightMin = 1e-30f, kBoundMax = 1e37f;
+
+__device__ __forceinline__ float boundFromWeight(float w, const WardRounding &r) {
+  return sqrtf(fminf(w, kBoundMax) * (1.0f - 2.0f * r.eps)) * (1.0f - 1e-6f);
+}
+
+// Adds (weight, rep) to a sorted list of kListK entries; returns the weight
+// that does not fit (+inf: none did fall out).
+__device__ __forceinline__ float keepLightest(float (&w)[kListK], int (&rep)[kListK], float nw,
+                                              int nrep) {
+#pragma unroll
+  for (int e = 0; e < kListK; ++e) {
+    const bool before = nw < w[e] || (nw == w[e] && (unsigned)nrep < (unsigned)rep[e]);
+    const float tw = before ? w[e] : nw;
+    const int tr = before ? rep[e] : nrep;
+    w[e] = before ? nw : w[e];
+    rep[e] = before ? nrep : rep[e];
+    nw = tw;
+    nrep = tr;
+  }
+  return nw;
+}
+
+__device__ __forceinline__ void storeList(const WardLists &out, int slot,
+                                          const float (&w)[kListK], const int (&rep)[kListK]) {
+#pragma unroll
+  for (int e = 0; e < kListK; ++e) {
+    out.rep[e * out.stride + slot] = rep[e];
+    out.weight[e * out.stride + slot] = w[e];
+  }
+}
+
+// After a round's merges: the lists, bounds and answers of the next round's
+// clusters (one thread per old slot that is not absorbed). First, clusters
+// outside a row's list may have merged: W(i, a u b) >= t (1 - 3 eps') with t =
+// min(W(i, a), W(i, b)) by the Lance-Williams form, since the computed w(a, b)
+// is at most the computed w(a, i); the stored centroid's offset takes at most
+// sqrt(2 n_i) delta off its square root. Then the row itself may have merged
+// with j at weight h: for c outside both lists the same form gives
+//   W(i u j, c) = [n_i W(i, c) + n_j W(j, c) + n_c (W(i, c) + W(j, c) - h)] /
+//                 (n_i + n_j + n_c),
+// a mean of (n_i b_i + n_j b_j) / (n_i + n_j) and b_i + b_j - h or more; the
+// second is the larger as a rule and weighs least for n_c = 1. flag <- whether
+// the row must search, cap <- the weight up to which it does (a partner at most
+// that heavy is known).
+__global__ void updateLists(WardLists in, WardLists out, const int *__restrict__ partner,
+                            const float *__restrict__ mergeWeight,
+                            const int *__restrict__ newIndex, const int *__restrict__ rep,
+                            const float *__restrict__ oldSize, int m,
+                            const int *__restrict__ slotOfRep, const float *__restrict__ cent,
+                            const float *__restrict__ size, const int *__restrict__ nextRep,
+                            const unsigned char *__restrict__ changed, int d, WardRounding r,
+                            unsigned long long *nearest, unsigned char *__restrict__ flag, float *__restrict__ cap) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= m)
+    return;
+  const int j = partner[i];
+  if (j >= 0 && rep[j] < rep[i])
+    return;
+  const int to = newIndex[i];
+  const float si = size[to];
+  const float *ci = cent + (size_t)to * d;
+  float w[kListK];
+  int reps[kListK];
+#pragma unroll
+  for (int e = 0; e < kListK; ++e) {
+    w[e] = INFINITY;
+    reps[e] = -1;
+  }
+  WardWeight weight;
+  auto stepped = [&](float root, float points) {
+    return root * (1.0f - 4.0f * r.eps) - 1.5f * sqrtf(2.0f * points) * r.delta;
+  };
+  float root = stepped(in.rootBound[i], j >= 0 ? oldSize[i] : si);
+  if (j >= 0) {
+    const float ni = oldSize[i], nj = oldSize[j];
+    const float rj = stepped(in.rootBound[j], nj);
+    const float bi = root > 0.0f ? root * root : 0.0f, bj = rj > 0.0f ? rj * rj : 0.0f;
+    const float near = bi * (ni / (ni + nj)) + bj * (nj / (ni + nj)); // no overflow
+    const float far = bi + bj - mergeWeight[to] * (1.0f + 2.0f * r.eps);
+    const float both =
+        far >= near ? near * (si / (si + 1.0f)) + far * (1.0f / (si + 1.0f)) : far;
+    root = stepped(sqrtf(fminf(fmaxf(both, 0.0f), kBoundMax)) * (1.0f - 1e-6f), si);
+  }
+  for (int side = 0; side < (j >= 0 ? 2 : 1); ++side) {
+    const int row = side ? j : i;
+    for (int e = 0; e < kListK; ++e) {
+      const int old = in.rep[e * in.stride + row];
+      if (old < 0)
+        break;
+      const int slot = slotOfRep[old];
+      if (slot == to)
+        continue; // the partner
+      const int now = nextRep[slot];
+      bool known = false;
+#pragma unroll
+      for (int q = 0; q < kListK; ++q)
+        known |= reps[q] == now;
+      if (known)
+        continue; // two members merged, or both rows list it
+      float nw = in.weight[e * in.stride + row];
+      if (j >= 0 || changed[slot]) {
+        // The pass's arithmetic: squared distance in feature order, weight.
+        const float *cj = cent + (size_t)slot * d;
+        float squared = 0.0f;
+        for (int k = 0; k < d; ++k) {
+          const float diff = ci[k] - cj[k];
+          squared = fmaf(diff, diff, squared);
+        }
+        nw = weight.weight(squared, si, size[slot]);
+      }
+      if (!(nw < INFINITY))
+        continue; // no edge
+      const float out = keepLightest(w, reps, nw > 0.0f ? nw : 0.0f, now);
+      if (out < INFINITY) // a partner leaves the list: the bound must cover it
+        root = fminf(root, boundFromWeight(out, r));
+    }
+  }
+  storeList(out, to, w, reps);
+  out.rootBound[to] = root;
+  // Computed weights outside the list are at least b (1 - eps).
+  const float bound = root * root * (1.0f - 2.0f * r.eps) * (1.0f - 1e-6f);
+  const bool settled = root > 0.0f && reps[0] >= 0 && w[0] > kWeightMin && w[0] < bound;
+  nearest[to] = reps[0] >= 0 ? packKey(w[0], (uint32_t)reps[0]) : kEmptyKey;
+  flag[to] = !settled;
+  float last = INFINITY;
+#pragma unroll
+  for (int e = 0; e < kListK; ++e)
+    last = reps[e] >= 0 ? w[e] : last;
+  // A list of one or two close partners would only be renewed as short.
+  cap[to] = fmaxf(last, w[0] * 1.1f);
+}
+
+// The searched rows' lists from the blocks' parts (one block of 128 threads per
+// row tile, thread = row): the kListK lightest of the parts' entries, the bound
+// from the last, the answer from the first by (weight, representative).
+// rowTiles: how many row tiles were searched (null: all of them, row tile I =
+// positions from I * 128 on); cap: the searched rows' cap, beyond which nothing
+// was evaluated (null: none). Every block of a searched row tile writes its
+// part: a split leaves every block at least kSplitTiles / 2 column tiles.
+__global__ void __launch_bounds__(kTile)
+    collectLists(const unsigned long long *__restrict__ parts, const int *__restrict__ rowTiles,
+                 const int *__restrict__ rowPos, int numBlocks, int numTiles, int m,
+                 const float *__restrict__ cap, WardLists out, WardRounding r,
+                 unsigned long long *__restrict__ nearest) {
+  const int tile = blockIdx.x, tiles = rowTiles ? *rowTiles : numBlocks;
+  if (tile >= tiles)
+    return;
+  const int pos = rowPos ? rowPos[(size_t)tile * kTile + threadIdx.x]
+                         : tile * kTile + (int)threadIdx.x;
+  if (pos < 0 || pos >= m)
+    return;
+  const int splits = rowTiles ? 1 << splitBitsFor(tiles, numBlocks, numTiles) : 1;
+  float w[kListK];
+  int reps[kListK];
+#pragma unroll
+  for (int e = 0; e < kListK; ++e) {
+    w[e] = INFINITY;
+    reps[e] = -1;
+  }
+  float least = cap ? fminf(cap[pos], kBoundMax) : kBoundMax; // of the weights left out
+  for (int s = 0; s < splits; ++s) {
+    const unsigned long long *part =
+        parts + (size_t)(s * tiles + tile) * kListK * kTile + threadIdx.x;
+    for (int e = 0; e < kListK; ++e) {
+      const unsigned long long key = part[(size_t)e * kTile];
+      const float v = listKeyValue(key);
+      if (!(v < INFINITY))
+        break;
+      if (e == kListK - 1)
+        least = fminf(least, v); // the block may have dropped others like it
+      least = fminf(least, keepLightest(w, reps, v, (int)(uint32_t)key));
+    }
+  }
+  storeList(out, pos, w, reps);
+  out.rootBound[pos] = boundFromWeight(least, r);
+  nearest[pos] = reps[0] >= 0 ? packKey(w[0], (uint32_t)reps[0]) : kEmptyKey;
 }
 
 __global__ void gatherClusters(const int *__restrict__ perm, const float *__restrict__ cent,
@@ -209,7 +446,10 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
   CUHC_TRY(st, index.build(devPoints, n, d, prune, s));
   DeviceBuffer<float> cent[2], sizeF[2];
   DeviceBuffer<int> size[2], rep[2];
-  DeviceBuffer<int> slotOfRep, partner, survive, newIndex, counter, error;
+  DeviceBuffer<int> slotOfRep, partner, survive, newIndex, counter, error, listRep[2];
+  DeviceBuffer<float> listWeight[2], rootBound[2], cap, mergeWeight;
+  DeviceBuffer<unsigned char> changed, searchFlag;
+  DeviceBuffer<unsigned long long> parts;
   DeviceBuffer<int> mergeU, mergeV;
   DeviceBuffer<float> mergeH;
   DeviceBuffer<unsigned long long> nearest, tiles;
@@ -218,7 +458,15 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
     CUHC_TRY(st, sizeF[b].allocate(paddedToTiles(n), s));
     CUHC_TRY(st, size[b].allocate(n, s));
     CUHC_TRY(st, rep[b].allocate(paddedToTiles(n), s));
+    CUHC_TRY(st, listRep[b].allocate((size_t)n * kListK, s));
+    CUHC_TRY(st, listWeight[b].allocate((size_t)n * kListK, s));
+    CUHC_TRY(st, rootBound[b].allocate(n, s));
   }
+  CUHC_TRY(st, cap.allocate(n, s));
+  CUHC_TRY(st, mergeWeight.allocate(n, s));
+  CUHC_TRY(st, changed.allocate(n, s));
+  CUHC_TRY(st, searchFlag.allocate(n, s));
+  CUHC_TRY(st, parts.allocate(paddedToTiles(n) * kListK, s));
   CUHC_TRY(st, slotOfRep.allocate(n, s));
   CUHC_TRY(st, partner.allocate(n, s));
   CUHC_TRY(st, survive.allocate(n, s));
@@ -248,6 +496,28 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
   noteLaunch();
   CUHC_TRY(st, cudaGetLastError());
 
+  auto listsOf = [&](int b) {
+    return WardLists{listRep[b].get(), listWeight[b].get(), rootBound[b].get(), (size_t)n};
+  };
+  WardRounding rounding{};
+  std::vector<float> boxLow(d), boxHigh(d);
+  CUHC_TRY(st, index.rootBox(boxLow, boxHigh));
+  if (st.ok()) {
+    const double u = std::ldexp(1.0, -24);
+    double square = 0.0;
+    for (int f = 0; f < d; ++f) {
+      const double extent = (double)boxHigh[f] - boxLow[f];
+      const double magnitude = std::max(std::fabs((double)boxLow[f]), std::fabs((double)boxHigh[f]));
+      const double e = u * (3.1 * extent + 1.1 * magnitude);
+      square += e * e;
+    }
+    rounding.eps = (float)(1.5 * (d + 12) * u);
+    rounding.delta = (float)(1.01 * std::sqrt(square));
+  }
+  // Merged centroids stay inside the points' box: the extent test holds for
+  // every round.
+  const bool screened =
+      st.ok() && useScreen<SqEuclideanMetric>(d, kListK) && index.extentsWithin(kScreenMaxExtent);
   std::vector<int> roundEnd;
   int m = n, merged = 0, cur = 0, rounds = 0;
   enum { kNone, kDense, kChain } tail = kNone;
@@ -277,24 +547,34 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
     p.nodeHigh = index.nodeHigh.get();
     p.nodeMinValue = index.nodeMinValue.get();
     p.prune = prune;
-    p.nearest = nearest.get();
-    p.compBest = nullptr;
+    p.k = kListK;
+    p.knnParts = parts.get();
     p.tilesComputed = tiles.get();
     p.error = error.get();
-  p.screenStats = screenCounters();
-  p.screenAudit = screenAuditWords();
+    p.screenStats = screenCounters();
+    p.screenAudit = screenAuditWords();
     WardWeight w;
     w.value = sizeF[cur].get();
+    if (rounds > 0 && m > kSearchAllBelow) {
+      bool ordered = false;
+      CUHC_TRY(st, index.selectRows(searchFlag.get(), nullptr, sizeF[cur].get(), &ordered));
+      p.rowPos = index.rowPos.get();
+      p.rowTiles = index.rowTiles.get();
+      p.rowTiled = index.rowTiled.get();
+      p.rowBoxLow = index.rowBoxLow.get();
+      p.rowBoxHigh = index.rowBoxHigh.get();
+      p.rowMinValue = index.rowMinValue.get();
+      p.rowPure = index.rowPure.get();
+      p.radius = cap.get();
+    }
     {
-      const bool screened =
-          useScreen<SqEuclideanMetric>(d, 0) && index.extentsWithin(kScreenMaxExtent);
       PassTimer timer(screened ? kTimerScreenPass : kTimerNearestPass, s);
       if (screened)
-        CUHC_TRY(st, (launchScreen<SqEuclideanMetric, WardWeight, false>(
+        CUHC_TRY(st, (launchScreen<SqEuclideanMetric, WardWeight, true>(
                          p, SqEuclideanMetric{}, w, index.kc, s)));
       else
-        CUHC_TRY(st, (launchPass<SqEuclideanMetric, WardWeight, false>(p, SqEuclideanMetric{}, w,
-                                                                       index.kc, s)));
+        CUHC_TRY(st, (launchPass<SqEuclideanMetric, WardWeight, true>(p, SqEuclideanMetric{}, w,
+                                                                      index.kc, s)));
       if (timer.start) {
         unsigned long long now = 0;
         cudaMemcpyAsync(&now, tiles.get(), sizeof(now), cudaMemcpyDeviceToHost, s);
@@ -302,6 +582,11 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
         tilesSoFar = now;
       }
     }
+    collectLists<<<index.numTiles, kTile, 0, s>>>(parts.get(), p.rowTiles, p.rowPos,
+                                                  index.numTiles, index.numTiles, m,
+                                                  p.radius, listsOf(cur), rounding,
+                                                  nearest.get());
+    noteLaunch();
     rnnPartners<<<blocks(m), 256, 0, s>>>(nearest.get(), slotOfRep.get(), rep[cur].get(), m,
                                           partner.get(), survive.get());
     noteLaunch();
@@ -311,8 +596,16 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
     rnnMerge<<<blocks((long long)m * d), 256, 0, s>>>(
         cent[cur].get(), size[cur].get(), rep[cur].get(), partner.get(), newIndex.get(), m, d,
         cent[nxt].get(), size[nxt].get(), sizeF[nxt].get(), rep[nxt].get(), slotOfRep.get(),
-        mergeU.get(), mergeV.get(), mergeH.get(), counter.get(), n - 1);
+        changed.get(), mergeWeight.get(), nearest.get(), mergeU.get(), mergeV.get(), mergeH.get(), counter.get(), n - 1);
     noteLaunch();
+    if (m > kSearchAllBelow) {
+      updateLists<<<blocks(m, 128), 128, 0, s>>>(
+          listsOf(cur), listsOf(nxt), partner.get(), mergeWeight.get(), newIndex.get(),
+          rep[cur].get(), sizeF[cur].get(), m, slotOfRep.get(), cent[nxt].get(),
+          sizeF[nxt].get(), rep[nxt].get(), changed.get(), d, rounding, nearest.get(),
+          searchFlag.get(), cap.get());
+      noteLaunch();
+    }
     CUHC_TRY(st, cudaGetLastError());
     int total = 0, passError = 0;
     CUHC_TRY(st, cudaMemcpyAsync(&total, counter.get(), sizeof(int), cudaMemcpyDeviceToHost, s));

@@ -27,6 +27,19 @@
 // other pair, and the epilogue takes a plain row minimum. Otherwise the
 // epilogue masks by component.
 //
+// Ward sizes. A pair weighs at most t only if s <= t (1 / s_i + 1 / s_j) / 2:
+// the bound depends on the column's cluster size, and with the smallest size
+// of the column tile in its place (as the box bounds use) a row of a round
+// with mixed sizes would recheck nearly every column of most tiles. The term
+// in s_j is a product of a row and a column value, so the MMA subtracts it: a
+// row whose threshold is capped by c from the start holds -c in one K slot,
+// the columns 1 / (2 s_j), both rounded up (c by 2^-8 more, far above the
+// accumulation's rounding of that product), and the row compares with
+// t / (2 s_i). The cap is a loose bound for many rows, so between phases the
+// row's current threshold takes its place. Ward of 200,000 x 32, all searches
+// after the first round: 290 ms without the term, 190 ms with the first cap
+// alone, 90 ms with the updates.
+//
 // Pipeline, warp-specialised, one row tile per block:
 //   producer warp 6: picks the next candidate tile (32 list entries per
 //     step) and lane 0 issues its bulk copies (raw coordinates + metadata)
@@ -82,6 +95,10 @@ constexpr int kBuilderThreads = 32 * kBuilderWarps;
 constexpr int kProducerWarp = 6; // picks candidate tiles and issues their bulk copies
 constexpr int kMmaWarp = 7;      // issues the MMAs
 constexpr int kFirstPhase = 64;  // tiles of a batch's first phase (then x8 per phase)
+// ... and of a pass with cluster sizes in the product, whose row thresholds go
+// into it between phases (then x4): 200,000 x 32 Ward passes in ms with first
+// phase and growth 16 x8 / 8 x2 / 4 x4 / 2 x2: 136 / 126 / 122 / 121.
+constexpr int kFirstSizedPhase = 4;
 constexpr float kIndicator = 0x1p90f;
 constexpr float kScreenAbsSlack = 0x1p-70f;
 constexpr float kScreenMaxExtent = 0x1p40f;
@@ -120,16 +137,6 @@ inline float screenMargin(int d, int kc) {
   const double centring = 4.0 * u;                      // a - c and b - c rounded
   const double reference = 2.02 * (d + 3) * u;          // the reference's FP32 chain
   return (float)(2.0 * (product + norms + mma + centring + reference));
-}
-
-// A k-NN list entry of the screened pass: value bits << 32 | position, so
-// that one 64-bit move carries both and keys order by value (values are
-// clamped at +0, so their bits order like the floats), then by position. An
-// empty entry holds +inf.
-constexpr unsigned long long kEmptyListKey = 0x7f800000ffffffffull;
-
-__device__ __forceinline__ float listKeyValue(unsigned long long key) {
-  return __uint_as_float((uint32_t)(key >> 32));
 }
 
 // Inserts `key` (its value below the k-th, whose entry leaves the list) into
@@ -284,12 +291,19 @@ __device__ __forceinline__ void storeOperandRow(float *op, int row, const float 
         make_float4(val[4 * q], val[4 * q + 1], val[4 * q + 2], val[4 * q + 3]);
 }
 
+// x >= 0 rounded up to TF32 (10 mantissa bits).
+__device__ __forceinline__ float tf32Up(float x) {
+  return __uint_as_float((__float_as_uint(x) + 0x1fffu) & ~0x1fffu);
+}
+
 // Row operand of row tile point i: [-2 x (KC), N hi, N lo, 1, 1, indicators]
-// (the factor -2, exact, sits on the side built once per row tile).
+// (the factor -2, exact, sits on the side built once per row tile). A nonzero
+// `extra` takes the first indicator slot.
 template <int KC>
 __device__ __forceinline__ void buildRowOperand(const float *sA, const float *centre, float scale,
                                                 int i, bool valid, int comp,
-                                                const ScreenSync &ss, float *opA) {
+                                                const ScreenSync &ss, float *opA,
+                                                float extra = 0.0f) {
   constexpr int kPad = screenKPad(KC), R = screenSlots(KC);
   float val[kPad];
   float n = 0.0f;
@@ -308,16 +322,19 @@ __device__ __forceinline__ void buildRowOperand(const float *sA, const float *ce
   for (int q = 0; q < R; ++q)
     val[KC + 4 + q] =
         (ss.oneHot && valid && q < ss.rowSetCount && comp == ss.rowSet[q]) ? kIndicator : 0.0f;
+  if (extra != 0.0f)
+    val[KC + 4] = extra;
   storeOperandRow<kPad>(opA, i, val);
 }
 
 // Column operand of staged point j: [y (KC), 1, 1, N hi, N lo, indicators];
-// the tile centre comes in registers.
+// the tile centre comes in registers. A nonzero `extra` takes the first
+// indicator slot.
 template <int KC>
 __device__ __forceinline__ void buildColumnOperand(const float *raw, const int *comp,
                                                    const float (&centre)[KC], float scale, int j,
                                                    bool oneHot, const ScreenSync &ss,
-                                                   float *opB) {
+                                                   float *opB, float extra = 0.0f) {
   constexpr int kPad = screenKPad(KC), R = screenSlots(KC);
   float val[kPad];
   float n = 0.0f;
@@ -336,6 +353,8 @@ __device__ __forceinline__ void buildColumnOperand(const float *raw, const int *
 #pragma unroll
   for (int q = 0; q < R; ++q)
     val[KC + 4 + q] = (oneHot && q < ss.rowSetCount && c == ss.rowSet[q]) ? 1.0f : 0.0f;
+  if (extra != 0.0f)
+    val[KC + 4] = extra;
   storeOperandRow<kPad>(opB, j, val);
 }
 
@@ -538,13 +557,15 @@ __global__ void __launch_bounds__(kThreads, 2)
   if (work.root < 0)
     return;
   const int leaf = p.leafOfTile[I];
-  const bool someRows = !kKnn && p.rowPos != nullptr;
+  const bool someRows = p.rowPos != nullptr;
   const int rowPure = (!kKnn && p.nodePure) ? (someRows ? p.rowPure[I] : p.nodePure[leaf]) : -1;
   const float rowMinValue =
       p.nodeMinValue ? (someRows ? p.rowMinValue[I] : p.nodeMinValue[leaf]) : 0.0f;
   const float slack = 1.0f - boxSlack(p.d);
   const bool useComp = !kKnn && p.component != nullptr;
-  const bool useValue = !kKnn && w.value != nullptr;
+  // k-NN by weight (the row itself left out) or by distance.
+  constexpr bool kWeighted = kKnn && !std::is_same<Weight, PlainWeight>::value;
+  const bool useValue = (!kKnn || kWeighted) && w.value != nullptr;
   const float scale = 1.0f - margin;
   constexpr bool kCos = std::is_same<Metric, CosineMetric>::value;
   // Cosine: 1 - e rounded down to TF32 (10 mantissa bits; the FP32 rounding of
@@ -641,12 +662,19 @@ __global__ void __launch_bounds__(kThreads, 2)
   tcgenFenceAfter();
   const uint32_t tmem = ss.tmemBase;
   const bool oneHot = ss.oneHot != 0;
+  // Ward: the row's cap goes into the product (header comment); sizes leave the
+  // indicator slots unused (every cluster its own component).
+  constexpr bool kSized = std::is_same<Weight, WardWeight>::value;
+  const float myCap = kSized && kKnn && mySearch && p.radius ? p.radius[myPos] : INFINITY;
+  const bool sizedPass = kSized && kKnn && p.radius != nullptr;
+  bool sized = kSized && myCap < 1e30f;
   float myNorm = 0.0f; // k-NN: the row's centred squared norm
   if (consumer) {
     if constexpr (kCos)
       buildRowOperandCosine<KC>(sA, myRow, mySearch, myComp, ss, opA);
     else
-      buildRowOperand<KC>(sA, centre, scale, myRow, mySearch, myComp, ss, opA);
+      buildRowOperand<KC>(sA, centre, scale, myRow, mySearch, myComp, ss, opA,
+                          sized ? -tf32Up(myCap * (1.0f + 0x1p-8f)) : 0.0f);
     if (kKnn) {
       float nrm = 0.0f;
 #pragma unroll
@@ -689,7 +717,9 @@ __global__ void __launch_bounds__(kThreads, 2)
     float thr;
     if (kKnn) {
       thr = listKeyValue(lists[myRow * p.k + p.k - 1]);
-      F = mySearch ? m.screenBound(thr) : -INFINITY;
+      if (kWeighted && mySearch && p.radius)
+        thr = fminf(thr, p.radius[myPos]);
+      F = mySearch ? m.screenBound(kWeighted ? w.distBound(thr, myVal) : thr) : -INFINITY;
     } else {
       thr = rowBest == kEmptyKey ? INFINITY : keyWeight(rowBest);
       if (compSlot) {
@@ -761,7 +791,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   unsigned long long computed = 0;
   // A pass over some of the rows has no self tile: the walk visits every
   // column tile.
-  bool selfPending = kKnn || (rowPure < 0 && !someRows);
+  bool selfPending = !someRows && (kKnn || rowPure < 0);
   bool overflow = false;
   bool dirty = false;                          // consumer: row filter may have tightened
   unsigned long long rechecks = 0, slowRows = 0; // consumer counters
@@ -835,8 +865,20 @@ __global__ void __launch_bounds__(kThreads, 2)
     // Phases of the batch: the producer issues phaseLimit tiles (kFirstPhase,
     // then eight times more each phase) and a sentinel; between phases every
     // warp tests the remaining candidates against the rows' current bounds.
-    int cursor = 0, phaseLimit = kFirstPhase;
+    int cursor = 0, phaseLimit = sizedPass ? kFirstSizedPhase : kFirstPhase;
     for (int phase = 0;; ++phase) {
+    if (sizedPass && (batch > 0 || phase > 0)) {
+      // The row's threshold takes the cap's place in the product (a looser cap
+      // would let every heavy-partner column through). No MMA is in flight.
+      if (consumer && mySearch && rowThr < 1e30f) {
+        *reinterpret_cast<float *>(reinterpret_cast<char *>(opA) + (myRow >> 3) * kSbo +
+                                   (myRow & 7) * 16 + (KC + 4) / 4 * 128) =
+            -tf32Up(rowThr * (1.0f + 0x1p-8f));
+        sized = true;
+      }
+      fenceProxyAsync();
+      __syncthreads();
+    }
     if (p.prune && (batch > 0 || phase > 0)) {
       for (int c = cursor + tid; c < len; c += kThreads)
         if (sh.listLb[c] < INFINITY && !rowsNeed(sh.listTile[c])) {
@@ -980,7 +1022,12 @@ __global__ void __launch_bounds__(kThreads, 2)
           for (int q = j; q < kTile; q += kBuilderThreads)
             if constexpr (kCos)
               buildColumnOperandCosine<KC>(raw, comp, cosC, q, oneHot, ss, b);
-            else
+            else if constexpr (kSized) {
+              // Slots past the clusters hold anything: size 1 does for them.
+              const float size = reinterpret_cast<const float *>(comp + kTile)[q];
+              buildColumnOperand<KC>(raw, comp, cen, scale, q, oneHot, ss, b,
+                                     tf32Up(size >= 1.0f ? 0.5f / size : 0.5f));
+            } else
               buildColumnOperand<KC>(raw, comp, cen, scale, q, oneHot, ss, b);
         }
         fenceProxyAsync();
@@ -1016,25 +1063,31 @@ __global__ void __launch_bounds__(kThreads, 2)
           // its bound -- the candidate bits of both chunks, built from the
           // same registers (no second read of tensor memory).
           float Fs = F + kScreenAbsSlack;
-          if constexpr (std::is_same<Weight, WardWeight>::value) {
-            // Ward: F assumes the lightest partner (size 1); the column tile's
-            // smallest cluster size s_min tightens it, since 2 si sj / (si + sj)
-            // grows with sj: a pair weighs <= thr only if its squared distance
-            // is <= thr (1/si + 1/s_min) / 2 (rounded up, as distBound).
+          if constexpr (kSized) {
+            // Ward. A capped row's product already holds the column's size.
+            // Otherwise F assumes the lightest partner (size 1); the column
+            // tile's smallest cluster size s_min tightens it, since 2 si sj /
+            // (si + sj) grows with sj: a pair weighs <= thr only if its squared
+            // distance is <= thr (1/si + 1/s_min) / 2 (rounded up, as distBound).
             float sMin = INFINITY;
+            if (__any_sync(0xffffffffu, !sized)) {
 #pragma unroll
-            for (int c = lane; c < kTile; c += 32)
-              if (J * kTile + c < p.n && cOrig[c] >= 0)
-                sMin = fminf(sMin, cVal[c]);
+              for (int c = lane; c < kTile; c += 32)
+                if (J * kTile + c < p.n && cOrig[c] >= 0)
+                  sMin = fminf(sMin, cVal[c]);
 #pragma unroll
-            for (int off = 16; off > 0; off /= 2)
-              sMin = fminf(sMin, __shfl_xor_sync(0xffffffffu, sMin, off));
-            if (F > -INFINITY && rowThr < INFINITY && sMin < INFINITY)
+              for (int off = 16; off > 0; off /= 2)
+                sMin = fminf(sMin, __shfl_xor_sync(0xffffffffu, sMin, off));
+            }
+            if (sized)
+              Fs = F > -INFINITY ? __fmul_ru(rowThr, 0.5f / myVal * 1.00002f) + kScreenAbsSlack
+                                 : -INFINITY;
+            else if (F > -INFINITY && rowThr < INFINITY && sMin < INFINITY)
               Fs = fminf(Fs, m.screenBound(__fmul_ru(
                                  rowThr, (1.0f / myVal + 1.0f / sMin) * 0.5f * 1.00001f)) +
                                  kScreenAbsSlack);
           }
-          if (kKnn && J == I && p.k <= kTile) {
+          if (kKnn && !kWeighted && J == I && p.k <= kTile) {
             // delta: 1.5 e (|x|^2 + |y|^2) bounds s - D' (the margin e is twice
             // the error bound); twice that, with the tile's largest norm.
             const float normMax = fmaxf(fmaxf(groupNorm[0], groupNorm[1]),
@@ -1127,7 +1180,19 @@ __global__ void __launch_bounds__(kThreads, 2)
               for (int k = 0; k < KC; ++k)
                 acc = m.accumulate(acc, sA[k * kTile + myRow], raw[k * kTile + jj]);
               ++rechecks;
-              if (kKnn) {
+              if (kWeighted) {
+                if (J * kTile + jj == myPos)
+                  continue; // the row itself
+                const float value = w.weight(m.finalize(acc), myVal, cVal[jj]);
+                if (value <= rowKth && value < INFINITY) {
+                  const unsigned long long key = packKey(value, (uint32_t)cOrig[jj]);
+                  if (key < list[p.k - 1]) {
+                    insertListKey(list, p.k, key);
+                    rowKth = listKeyValue(list[p.k - 1]);
+                    dirty = true;
+                  }
+                }
+              } else if (kKnn) {
                 const float value = J * kTile + jj == myPos ? 0.0f : fmaxf(m.finalize(acc), 0.0f);
                 // Offer to the row's list (the k-th value kept in a register):
                 // a value below the k-th enters, and the boundary-tie flag
@@ -1199,7 +1264,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     cursor = ss.cursor;
     if (ss.failed || ss.batchDone)
       break;
-    phaseLimit *= 8;
+    phaseLimit *= sizedPass ? 4 : 8;
     } // phases
     ++batch;
     if (ss.failed)
@@ -1216,7 +1281,10 @@ __global__ void __launch_bounds__(kThreads, 2)
       mbarrierWait(&ss.rawFull[o % S], (o / S) & 1);
   if (mmaThread && ss.failed && lastCommit >= 0)
     mbarrierWait(&ss.mmaFull[lastCommit & 1], (lastCommit >> 1) & 1);
-  if (consumer && myPos >= 0) {
+  if (kWeighted && consumer)
+    for (int e = 0; e < p.k; ++e)
+      p.knnParts[((size_t)blockIdx.x * p.k + e) * kTile + myRow] = lists[myRow * p.k + e];
+  if (consumer && myPos >= 0 && !kWeighted) {
     if (kKnn) {
       const int rank = myValid ? (p.coreRank ? p.coreRank[myPos] : p.k) : 0;
       p.core[myPos] = rank > 0 ? listKeyValue(lists[myRow * p.k + rank - 1]) : 0.0f;

@@ -529,13 +529,21 @@ int SpatialIndex::updateMinValues(const float *values) {
   return (int)cudaGetLastError();
 }
 
+int SpatialIndex::rootBox(std::vector<float> &low, std::vector<float> &high) {
+  StatusChain st;
+  low.resize(d);
+  high.resize(d);
+  CUHC_TRY(st, cudaMemcpyAsync(low.data(), nodeLow.get(), d * sizeof(float),
+                               cudaMemcpyDeviceToHost, stream));
+  CUHC_TRY(st, cudaMemcpyAsync(high.data(), nodeHigh.get(), d * sizeof(float),
+                               cudaMemcpyDeviceToHost, stream));
+  CUHC_TRY(st, cudaStreamSynchronize(stream));
+  return st.code;
+}
+
 bool SpatialIndex::extentsWithin(float limit) {
-  std::vector<float> low(d), high(d);
-  if (cudaMemcpyAsync(low.data(), nodeLow.get(), d * sizeof(float), cudaMemcpyDeviceToHost,
-                      stream) != cudaSuccess ||
-      cudaMemcpyAsync(high.data(), nodeHigh.get(), d * sizeof(float), cudaMemcpyDeviceToHost,
-                      stream) != cudaSuccess ||
-      cudaStreamSynchronize(stream) != cudaSuccess)
+  std::vector<float> low, high;
+  if (rootBox(low, high) != 0)
     return false;
   for (int f = 0; f < d; ++f)
     if (!(high[f] - low[f] <= limit)) // NaN fails too
@@ -815,7 +823,7 @@ __global__ void __launch_bounds__(kTile)
 int SpatialIndex::selectRows(const unsigned char *flag, const int *component,
                              const float *values, bool *ordered) {
   StatusChain st;
-  const bool order = numInstances > 1 || orderMatters();
+  const bool order = numInstances > 1 || (tileWorkValid && orderMatters());
   *ordered = order;
   if (order)
     CUHC_TRY(st, allocateTileOrder());

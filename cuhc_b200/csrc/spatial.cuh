@@ -100,6 +100,8 @@ struct SpatialIndex {
   // finite and at most `limit`. Copies the root box to the host and waits
   // for the index stream.
   bool extentsWithin(float limit);
+  // The root box (d floats each). Waits for the index stream.
+  int rootBox(std::vector<float> &low, std::vector<float> &high);
   // Whether every point's squared norm is 0 or within [low, high] (the
   // cosine screen's range). Computed once per index; retile resets it.
   bool normsWithin(float low, float high);
