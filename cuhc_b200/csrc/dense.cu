@@ -9,17 +9,27 @@
 // was a or b and got farther. The reference does the same three steps per
 // merge (linkage.cuh:86-268) with the same tie rules and formulas.
 //
-// B200 shape: the three kernels of a step are captured once into a CUDA
-// graph of kStepsPerGraph steps; the step counter lives on the device, so the
-// graph is replayed ceil((n-1) / kStepsPerGraph) times with no host work in
-// between and surplus steps exit at once.
+// B200 shape: a merge is a chain of short dependent steps, so all of them run
+// in one thread-block cluster that stays resident for the whole tree. The slots
+// are dealt out over its blocks, whose shared memory holds their nearest
+// neighbours and sizes; per merge the blocks exchange their minima through
+// distributed shared memory around one cluster barrier, and read and write the
+// matrix through L2. A merge is bound by that chain's latency (reduction,
+// barrier, two row reads, the rescans): 5 us at 300 and 1,000 points, 6.3 at
+// 3,001 and 20 at 16,000, where a captured graph of four kernels per merge, each
+// a launch and a pass through memory, took 13, 12, 11 and 25 us.
 #include "profiling.cuh"
 #include "rnn.cuh"
 
+#include <algorithm>
 #include <vector>
+
+#include <cooperative_groups.h>
 
 #include "metrics.cuh"
 #include "pairwise.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace cuhc {
 
@@ -28,23 +38,20 @@ int pairwiseIntoMatrix(const float *points, int n, int d, int metricId, float p,
 
 namespace {
 
-constexpr int kReduceThreads = 1024, kRescanThreads = 256, kStepsPerGraph = 64;
+constexpr int kRescanThreads = 256;
+// Blocks of the cluster (the portable limit) and their threads; a block takes
+// fewer than kMinSlots slots only when it is alone.
+constexpr int kClusterBlocks = 8, kMergeThreads = 512, kMinSlots = 128;
+// Dynamic shared memory a block of the cluster may take (227 KiB per block,
+// less its static arrays).
+constexpr size_t kDenseShared = 224 * 1024;
 enum LinkageKind : int { kSingleL = 0, kCompleteL = 1, kAverageL = 2, kWardL = 3 };
 
+// One merge: slots a < b at `distance` into a cluster of `size` points.
 struct MergeRecord {
   int a, b;
   float distance;
-  int sizeA, sizeB;
-};
-
-struct DenseState {
-  float *dist;
-  float *nearDist;
-  int *nearSlot, *size, *id, *rescan, *rescanCount, *step;
-  unsigned char *active;
-  MergeRecord *merge;
-  double *tree;
-  int n, firstNewId, linkage;
+  int size;
 };
 
 // Distance from the merged cluster (a u b) to k from the old distances, in
@@ -71,35 +78,18 @@ __device__ __forceinline__ bool lessLoc(float da, int ia, float db, int ib) {
   return da < db || (da == db && ia < ib);
 }
 
-__global__ void denseInit(DenseState s, const int *initialSize, const int *initialId) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= s.n)
-    return;
-  s.dist[(size_t)i * s.n + i] = INFINITY;
-  s.size[i] = initialSize ? initialSize[i] : 1;
-  s.id[i] = initialId ? initialId[i] : i;
-  s.active[i] = 1;
-  s.rescan[i] = i;
-  if (i == 0) {
-    *s.rescanCount = s.n;
-    *s.step = 0;
-  }
-}
-
-// Nearest active slot of every listed row (retired columns hold +inf).
-__global__ void __launch_bounds__(kRescanThreads) denseRescan(DenseState s) {
-  if (*s.step >= s.n - 1 && s.n > 1 && *s.step > 0) // past the last merge
-    return;
+// Nearest other slot of every row.
+__global__ void __launch_bounds__(kRescanThreads)
+    denseNearest(float *__restrict__ dist, int n, float *__restrict__ nearDist,
+                 int *__restrict__ nearSlot) {
   __shared__ float wd[kRescanThreads / 32];
   __shared__ int ws[kRescanThreads / 32];
-  const int count = *s.rescanCount;
-  for (int item = blockIdx.x; item < count; item += gridDim.x) {
-    const int row = s.rescan[item];
-    const float *r = s.dist + (size_t)row * s.n;
+  for (int row = blockIdx.x; row < n; row += gridDim.x) {
+    const float *r = dist + (size_t)row * n;
     float best = INFINITY;
     int slot = 0x7fffffff;
-    for (int c = threadIdx.x; c < s.n; c += kRescanThreads)
-      if (lessLoc(r[c], c, best, slot)) {
+    for (int c = threadIdx.x; c < n; c += kRescanThreads)
+      if (c != row && lessLoc(r[c], c, best, slot)) {
         best = r[c];
         slot = c;
       }
@@ -122,108 +112,229 @@ __global__ void __launch_bounds__(kRescanThreads) denseRescan(DenseState s) {
           best = wd[w];
           slot = ws[w];
         }
-      s.nearDist[row] = best;
-      s.nearSlot[row] = slot;
+      nearDist[row] = best;
+      nearSlot[row] = slot;
     }
     __syncthreads();
   }
 }
 
-// One block: the closest pair, the tree row, the bookkeeping of slot a.
-__global__ void __launch_bounds__(kReduceThreads) denseClosestPair(DenseState s) {
-  const int step = *s.step;
-  if (step >= s.n - 1)
-    return;
-  __shared__ float wd[kReduceThreads / 32];
-  __shared__ int ws[kReduceThreads / 32];
-  float best = INFINITY;
-  int slot = 0x7fffffff;
-  for (int i = threadIdx.x; i < s.n; i += kReduceThreads)
-    if (lessLoc(s.nearDist[i], i, best, slot)) {
-      best = s.nearDist[i];
-      slot = i;
-    }
-  for (int off = 16; off > 0; off /= 2) {
-    const float od = __shfl_xor_sync(0xffffffffu, best, off);
-    const int os = __shfl_xor_sync(0xffffffffu, slot, off);
-    if (lessLoc(od, os, best, slot)) {
-      best = od;
-      slot = os;
-    }
+// (distance, slot) as a key whose unsigned order is lessLoc's (-0 as +0).
+__device__ __forceinline__ unsigned long long locKey(float d, int slot) {
+  return ((unsigned long long)orderedBits(d + 0.0f) << 32) | (unsigned int)slot;
+}
+
+__device__ __forceinline__ unsigned long long minKey(unsigned long long x, unsigned long long y) {
+  return y < x ? y : x;
+}
+
+__device__ __forceinline__ unsigned long long warpMinKey(unsigned long long key) {
+#pragma unroll
+  for (int off = 16; off > 0; off /= 2)
+    key = minKey(key, __shfl_xor_sync(0xffffffffu, key, off));
+  return key;
+}
+
+// What a block tells the others per merge: its closest slot with its nearest
+// slot, and its part of the last merged row's nearest slot.
+struct MergeNote {
+  unsigned long long best, row;
+  int other, unused;
+};
+
+// The nearest active slot of row `r`, over `lanes` threads of which this is
+// number `lane`: the thread's part (the caller reduces).
+__device__ __forceinline__ unsigned long long scanRow(const float *__restrict__ r, int n, int self,
+                                                      const unsigned int *active, int lane,
+                                                      int lanes) {
+  unsigned long long best = kEmptyKey;
+#pragma unroll 8
+  for (int c = lane; c < n; c += lanes) {
+    const float d = __ldcg(r + c);
+    // Same as lessLoc from (+inf, INT_MAX): NaN never enters.
+    if (c != self && ((active[c >> 5] >> (c & 31)) & 1u) && d <= INFINITY)
+      best = minKey(best, locKey(d, c));
   }
-  if ((threadIdx.x & 31) == 0) {
-    wd[threadIdx.x >> 5] = best;
-    ws[threadIdx.x >> 5] = slot;
+  return best;
+}
+
+// All merges, in one cluster. Block c owns the slots [c * perBlock, ...): their
+// nearest slots and sizes live in its shared memory, and only it rescans their
+// rows; `active` is a copy of the live slots per block.
+//
+// Per merge: (1) every block reduces its closest slot and its part of the last
+// merged row's nearest; (2) they go to every block's notes, and one cluster
+// barrier later (notes alternate between two buffers) every block knows the
+// closest pair a < b; (3) each thread updates its slots k: distance to the
+// merged cluster into row a and column a, and k's nearest slot -- kept, taken,
+// or lost, when it was a or b and got farther; (4) lost ones are rescanned. The
+// barrier also publishes the matrix entries that a later merge reads in other
+// blocks (loads bypass L1). A size changes only after the barrier that follows
+// its merge; until then the readers know it as the last merge's.
+__global__ void __launch_bounds__(kMergeThreads)
+    denseMerges(float *__restrict__ dist, int n, int perBlock, int linkage,
+                const float *__restrict__ nearDist0, const int *__restrict__ nearSlot0,
+                const int *__restrict__ initialSize, float *__restrict__ spill,
+                MergeRecord *__restrict__ merges, int *__restrict__ mergeCount) {
+  extern __shared__ __align__(16) unsigned char dense_shared[];
+  __shared__ MergeNote notes[2][kClusterBlocks];
+  __shared__ unsigned long long warpBest[kMergeThreads / 32], warpRow[kMergeThreads / 32];
+  __shared__ int lostCount;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), blocks = (int)cluster.num_blocks();
+  int *size = reinterpret_cast<int *>(dense_shared);
+  unsigned int *active = reinterpret_cast<unsigned int *>(size + perBlock);
+  // The block's own: in shared memory, or past its reach in `spill`.
+  float *nearDist = spill ? spill + (size_t)rank * 3 * perBlock
+                          : reinterpret_cast<float *>(active + (n + 31) / 32);
+  int *nearSlot = reinterpret_cast<int *>(nearDist + perBlock);
+  int *lost = nearSlot + perBlock;
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int kWarps = kMergeThreads / 32;
+  const int first = rank * perBlock, slots = max(0, min(perBlock, n - first));
+  for (int i = tid; i < slots; i += kMergeThreads) {
+    nearDist[i] = nearDist0[first + i];
+    nearSlot[i] = nearSlot0[first + i];
+    size[i] = initialSize ? initialSize[first + i] : 1;
   }
+  for (int w = tid; w < (n + 31) / 32; w += kMergeThreads)
+    active[w] = n - w * 32 >= 32 ? 0xffffffffu : (1u << (n - w * 32)) - 1;
+  if (tid == 0)
+    lostCount = 0;
   __syncthreads();
-  if (threadIdx.x != 0)
-    return;
-  for (int w = 1; w < kReduceThreads / 32; ++w)
-    if (lessLoc(wd[w], ws[w], best, slot)) {
-      best = wd[w];
-      slot = ws[w];
-    }
-  if (!(best < INFINITY) || slot < 0 || slot >= s.n) { // no finite pair left: stop
-    *s.step = s.n;
-    return;
-  }
-  const int other = s.nearSlot[slot];
-  const int a = min(slot, other), b = max(slot, other);
-  const int na = s.size[a], nb = s.size[b];
-  const int ia = s.id[a], ib = s.id[b];
-  *s.merge = MergeRecord{a, b, best, na, nb};
-  double *row = s.tree + (size_t)step * 4;
-  row[0] = min(ia, ib);
-  row[1] = max(ia, ib);
-  row[2] = best;
-  row[3] = na + nb;
-  s.size[a] = na + nb;
-  s.id[a] = s.firstNewId + step;
-  s.active[b] = 0;
-  s.nearDist[b] = INFINITY;
-  *s.rescanCount = 0;
-}
 
-// One thread per slot k: the Lance-Williams distance of the merged cluster,
-// and whether k's cached nearest is still valid.
-__global__ void denseMerge(DenseState s) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  const int step = *s.step;
-  if (k >= s.n || step >= s.n - 1 || !s.active[k])
-    return;
-  const MergeRecord mg = *s.merge;
-  const int a = mg.a, b = mg.b;
-  const size_t n = s.n;
-  if (k == a) {
-    s.dist[(size_t)a * n + b] = INFINITY;
-    s.rescan[atomicAdd(s.rescanCount, 1)] = a;
-    return;
-  }
-  const float nd = (float)lanceWilliams(s.linkage, s.dist[(size_t)a * n + k],
-                                        s.dist[(size_t)b * n + k], mg.distance, mg.sizeA,
-                                        mg.sizeB, s.size[k]);
-  s.dist[(size_t)a * n + k] = nd;
-  s.dist[(size_t)k * n + a] = nd;
-  s.dist[(size_t)k * n + b] = INFINITY;
-  const int near = s.nearSlot[k];
-  if (near == a || near == b) {
-    if (nd <= s.nearDist[k]) {
-      s.nearDist[k] = nd;
-      s.nearSlot[k] = a;
-    } else {
-      s.rescan[atomicAdd(s.rescanCount, 1)] = k;
+  unsigned long long rowPart = kEmptyKey; // this thread's part of the last merged row
+  int lastA = -1, lastSize = 0, step = 0;
+  for (; step < n - 1; ++step) {
+    // (1) The block's closest slot (the last merged row's is not known yet).
+    unsigned long long best = kEmptyKey;
+    for (int i = tid; i < slots; i += kMergeThreads)
+      if (first + i != lastA && nearDist[i] < INFINITY)
+        best = minKey(best, locKey(nearDist[i], first + i));
+    best = warpMinKey(best);
+    rowPart = warpMinKey(rowPart);
+    if (lane == 0) {
+      warpBest[warp] = best;
+      warpRow[warp] = rowPart;
     }
-  } else if (nd < s.nearDist[k]) {
-    s.nearDist[k] = nd;
-    s.nearSlot[k] = a;
+    __syncthreads();
+    // (2) To every block.
+    if (warp == 0) {
+      best = warpMinKey(lane < kWarps ? warpBest[lane] : kEmptyKey);
+      rowPart = warpMinKey(lane < kWarps ? warpRow[lane] : kEmptyKey);
+      if (lane < blocks) {
+        MergeNote note;
+        note.best = best;
+        note.row = rowPart;
+        note.other = best == kEmptyKey ? -1 : nearSlot[(int)(uint32_t)best - first];
+        note.unused = 0;
+        *cluster.map_shared_rank(&notes[step & 1][rank], lane) = note;
+      }
+    }
+    cluster.sync();
+    MergeNote note;
+    note.best = note.row = kEmptyKey;
+    note.other = -1;
+    if (lane < blocks)
+      note = notes[step & 1][lane];
+    const unsigned long long blockBest = note.best, row = warpMinKey(note.row);
+    best = warpMinKey(blockBest);
+    const unsigned from = __ballot_sync(0xffffffffu, blockBest == best);
+    int other = __shfl_sync(0xffffffffu, note.other, __ffs(from) - 1);
+    if (lastA >= 0) {
+      const float d = row == kEmptyKey ? INFINITY : orderedFloat((uint32_t)(row >> 32));
+      const int slot = row == kEmptyKey ? 0x7fffffff : (int)(uint32_t)row;
+      if (d < INFINITY && locKey(d, lastA) < best) {
+        best = locKey(d, lastA);
+        other = slot;
+      }
+      if (lastA >= first && lastA < first + slots && tid == 0) {
+        nearDist[lastA - first] = d;
+        nearSlot[lastA - first] = slot;
+        size[lastA - first] = lastSize;
+      }
+    }
+    if (best == kEmptyKey)
+      break; // no finite pair left
+    const float distance = orderedFloat((uint32_t)(best >> 32));
+    const int closest = (int)(uint32_t)best;
+    const int a = min(closest, other), b = max(closest, other);
+    auto sizeOf = [&](int slot) {
+      return slot == lastA ? lastSize
+                           : *cluster.map_shared_rank(&size[slot % perBlock], slot / perBlock);
+    };
+    const int sizeA = sizeOf(a), sizeB = sizeOf(b);
+    if (rank == 0 && tid == 0)
+      merges[step] = MergeRecord{a, b, distance, sizeA + sizeB};
+    // Everyone has read the old nearest slots and the last row's is stored.
+    __syncthreads();
+    if (tid == 0) {
+      active[b >> 5] &= ~(1u << (b & 31));
+      lostCount = 0;
+    }
+    __syncthreads();
+    // (3) The slots' distances to the merged cluster.
+    rowPart = kEmptyKey;
+    for (int i = tid; i < slots; i += kMergeThreads) {
+      const int k = first + i;
+      if (k == b)
+        nearDist[i] = INFINITY;
+      if (k == a || !((active[k >> 5] >> (k & 31)) & 1u))
+        continue;
+      const float nd = (float)lanceWilliams(
+          linkage, __ldcg(dist + (size_t)a * n + k), __ldcg(dist + (size_t)b * n + k), distance,
+          sizeA, sizeB, k == lastA ? lastSize : size[i]);
+      dist[(size_t)a * n + k] = nd;
+      dist[(size_t)k * n + a] = nd;
+      if (nd <= INFINITY)
+        rowPart = minKey(rowPart, locKey(nd, k));
+      const int near = nearSlot[i];
+      if (near == a || near == b) {
+        if (nd <= nearDist[i]) {
+          nearDist[i] = nd;
+          nearSlot[i] = a;
+        } else {
+          lost[atomicAdd(&lostCount, 1)] = i;
+        }
+      } else if (nd < nearDist[i]) {
+        nearDist[i] = nd;
+        nearSlot[i] = a;
+      }
+    }
+    __syncthreads();
+    // (4) Rescans: the block's warps shared out over the lost rows (a warp per
+    // row took 15 us per merge at 3,001 points).
+    const int count = lostCount;
+    int perRow = kWarps; // warps per row, a power of two
+    while (perRow > 1 && perRow * count > kWarps)
+      perRow /= 2;
+    for (int base = 0; base < count; base += kWarps / perRow) {
+      const int q = base + warp / perRow, part = warp % perRow;
+      unsigned long long key = kEmptyKey;
+      if (q < count) {
+        const int row = first + lost[q];
+        key = warpMinKey(scanRow(dist + (size_t)row * n, n, row, active, part * 32 + lane,
+                                 perRow * 32));
+      }
+      if (lane == 0)
+        warpBest[warp] = key;
+      __syncthreads();
+      if (q < count && part == 0 && lane == 0) {
+        for (int w = 1; w < perRow; ++w)
+          key = minKey(key, warpBest[warp + w]);
+        nearDist[lost[q]] = key == kEmptyKey ? INFINITY : orderedFloat((uint32_t)(key >> 32));
+        nearSlot[lost[q]] = key == kEmptyKey ? 0x7fffffff : (int)(uint32_t)key;
+      }
+      __syncthreads();
+    }
+    __syncthreads();
+    lastA = a;
+    lastSize = sizeA + sizeB;
   }
-}
-
-// Next step; stays at n - 1 after the last merge, and at n after an early
-// stop (no finite pair left), which the host reports as an error.
-__global__ void denseAdvance(DenseState s) {
-  if (*s.step < s.n - 1)
-    ++*s.step;
+  if (rank == 0 && tid == 0)
+    *mergeCount = step;
+  cluster.sync(); // no block's shared memory goes while another may read it
 }
 
 __global__ void wardTransform(float *dist, const int *size, int m) {
@@ -238,74 +349,82 @@ __global__ void wardTransform(float *dist, const int *size, int m) {
 } // namespace
 
 int denseLinkageFromMatrix(float *distances, const int *initialSize, const int *initialId,
-                           int firstNewId, int m, int linkageId, double *deviceTree,
+                           int firstNewId, int m, int linkageId, double *hostTree,
                            cudaStream_t s) {
   if (m < 2)
     return 0;
   StatusChain st;
   DeviceBuffer<float> nearDist;
-  DeviceBuffer<int> ints;
-  DeviceBuffer<unsigned char> active;
-  DeviceBuffer<MergeRecord> merge;
+  DeviceBuffer<int> nearSlot, mergeCount;
+  DeviceBuffer<MergeRecord> merges;
   CUHC_TRY(st, nearDist.allocate(m, s));
-  CUHC_TRY(st, ints.allocate((size_t)4 * m + 2, s));
-  CUHC_TRY(st, active.allocate(m, s));
-  CUHC_TRY(st, merge.allocate(1, s));
+  CUHC_TRY(st, nearSlot.allocate(m, s));
+  CUHC_TRY(st, mergeCount.allocate(1, s));
+  CUHC_TRY(st, merges.allocate(m - 1, s));
   if (!st.ok())
     return st.code;
-  DenseState ds{};
-  ds.dist = distances;
-  ds.nearDist = nearDist.get();
-  ds.nearSlot = ints.get();
-  ds.size = ints.get() + m;
-  ds.id = ints.get() + 2 * m;
-  ds.rescan = ints.get() + 3 * m;
-  ds.rescanCount = ints.get() + 4 * m;
-  ds.step = ints.get() + 4 * m + 1;
-  ds.active = active.get();
-  ds.merge = merge.get();
-  ds.tree = deviceTree;
-  ds.n = m;
-  ds.firstNewId = firstNewId;
-  ds.linkage = linkageId;
-  const int perSlot = (m + 255) / 256;
   int device = 0, sms = 0;
   cudaGetDevice(&device);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  denseInit<<<perSlot, 256, 0, s>>>(ds, initialSize, initialId);
-  noteLaunch();
-  denseRescan<<<4 * sms, kRescanThreads, 0, s>>>(ds);
+  denseNearest<<<std::min(m, 8 * sms), kRescanThreads, 0, s>>>(distances, m, nearDist.get(),
+                                                               nearSlot.get());
   noteLaunch();
   CUHC_TRY(st, cudaGetLastError());
-  // One graph of kStepsPerGraph merges, replayed.
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  CUHC_TRY(st, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-  if (st.ok()) {
-    for (int i = 0; i < kStepsPerGraph; ++i) {
-      denseClosestPair<<<1, kReduceThreads, 0, s>>>(ds);
-      denseMerge<<<perSlot, 256, 0, s>>>(ds);
-      denseRescan<<<4 * sms, kRescanThreads, 0, s>>>(ds);
-      denseAdvance<<<1, 1, 0, s>>>(ds);
-    }
-    CUHC_TRY(st, cudaStreamEndCapture(s, &graph));
+  int blocks = 1;
+  while (blocks < kClusterBlocks && m > blocks * kMinSlots)
+    blocks *= 2;
+  const int perBlock = (m + blocks - 1) / blocks;
+  const size_t own = (size_t)3 * perBlock;
+  size_t shared = ((size_t)perBlock + (m + 31) / 32 + own) * sizeof(int);
+  DeviceBuffer<float> spill;
+  if (shared > kDenseShared) {
+    CUHC_TRY(st, spill.allocate(own * blocks, s));
+    shared -= own * sizeof(int);
   }
-  CUHC_TRY(st, cudaGraphInstantiate(&exec, graph, 0));
-  const int replays = (m - 1 + kStepsPerGraph - 1) / kStepsPerGraph;
-  for (int r = 0; r < replays && st.ok(); ++r) {
-    CUHC_TRY(st, cudaGraphLaunch(exec, s));
-    noteLaunch(4 * kStepsPerGraph);
-  }
+  CUHC_TRY(st, cudaFuncSetAttribute(denseMerges, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)shared));
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(blocks);
+  config.blockDim = dim3(kMergeThreads);
+  config.dynamicSmemBytes = shared;
+  config.stream = s;
+  cudaLaunchAttribute attribute{};
+  attribute.id = cudaLaunchAttributeClusterDimension;
+  attribute.val.clusterDim.x = blocks;
+  attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  CUHC_TRY(st, cudaLaunchKernelEx(&config, denseMerges, distances, m, perBlock, linkageId,
+                                  (const float *)nearDist.get(), (const int *)nearSlot.get(),
+                                  initialSize, spill.get(), merges.get(), mergeCount.get()));
+  noteLaunch();
+  std::vector<MergeRecord> host(m - 1);
+  std::vector<int> id(m);
+  int count = 0;
+  CUHC_TRY(st, cudaMemcpyAsync(host.data(), merges.get(), merges.bytes(), cudaMemcpyDeviceToHost,
+                               s));
+  CUHC_TRY(st, cudaMemcpyAsync(&count, mergeCount.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
+  if (initialId)
+    CUHC_TRY(st, cudaMemcpyAsync(id.data(), initialId, m * sizeof(int), cudaMemcpyDeviceToHost,
+                                 s));
+  else
+    for (int i = 0; i < m; ++i)
+      id[i] = i;
   CUHC_TRY(st, cudaStreamSynchronize(s));
-  if (exec)
-    cudaGraphExecDestroy(exec);
-  if (graph)
-    cudaGraphDestroy(graph);
-  int step = 0;
-  CUHC_TRY(st, cudaMemcpy(&step, ds.step, sizeof(int), cudaMemcpyDeviceToHost));
-  if (st.ok() && step != m - 1)
+  if (st.ok() && count != m - 1)
     st(kErrorNonFinite);
-  return st.code;
+  if (!st.ok())
+    return st.code;
+  for (int step = 0; step < m - 1; ++step) {
+    const MergeRecord &merge = host[step];
+    double *row = hostTree + (size_t)step * 4;
+    row[0] = std::min(id[merge.a], id[merge.b]);
+    row[1] = std::max(id[merge.a], id[merge.b]);
+    row[2] = merge.distance;
+    row[3] = merge.size;
+    id[merge.a] = firstNewId + step;
+  }
+  return 0;
 }
 
 int denseLinkage(const float *devPoints, int n, int d, int metricId, float p, int linkageId,
@@ -314,13 +433,9 @@ int denseLinkage(const float *devPoints, int n, int d, int metricId, float p, in
     return 0;
   StatusChain st;
   DeviceBuffer<float> dist;
-  DeviceBuffer<double> tree;
   CUHC_TRY(st, dist.allocate((size_t)n * n, s));
-  CUHC_TRY(st, tree.allocate((size_t)(n - 1) * 4, s));
   CUHC_TRY(st, pairwiseIntoMatrix(devPoints, n, d, metricId, p, dist.get(), s));
-  CUHC_TRY(st, denseLinkageFromMatrix(dist.get(), nullptr, nullptr, n, n, linkageId, tree.get(), s));
-  CUHC_TRY(st, cudaMemcpyAsync(hostTree, tree.get(), tree.bytes(), cudaMemcpyDeviceToHost, s));
-  CUHC_TRY(st, cudaStreamSynchronize(s));
+  CUHC_TRY(st, denseLinkageFromMatrix(dist.get(), nullptr, nullptr, n, n, linkageId, hostTree, s));
   return st.code;
 }
 
@@ -329,17 +444,14 @@ int denseOnWardMatrix(const float *centroids, const int *sizes, const int *reps,
                       std::vector<float> &h) {
   StatusChain st;
   DeviceBuffer<float> dist;
-  DeviceBuffer<double> tree;
   CUHC_TRY(st, dist.allocate((size_t)m * m, s));
-  CUHC_TRY(st, tree.allocate((size_t)(m - 1) * 4, s));
   CUHC_TRY(st, pairwiseIntoMatrix(centroids, m, d, kSqEuclidean, 2.0f, dist.get(), s));
   wardTransform<<<(int)(((long long)m * m + 255) / 256), 256, 0, s>>>(dist.get(), sizes, m);
   noteLaunch();
   CUHC_TRY(st, cudaGetLastError());
-  CUHC_TRY(st, denseLinkageFromMatrix(dist.get(), sizes, reps, numPoints, m, kWardL, tree.get(), s));
   std::vector<double> host((size_t)(m - 1) * 4);
-  CUHC_TRY(st, cudaMemcpyAsync(host.data(), tree.get(), tree.bytes(), cudaMemcpyDeviceToHost, s));
-  CUHC_TRY(st, cudaStreamSynchronize(s));
+  CUHC_TRY(st, denseLinkageFromMatrix(dist.get(), sizes, reps, numPoints, m, kWardL, host.data(),
+                                      s));
   if (!st.ok())
     return st.code;
   // Tree ids -> representative points: a new cluster is represented by the

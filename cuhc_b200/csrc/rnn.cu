@@ -50,7 +50,7 @@ int denseOnWardMatrix(const float *centroids, const int *sizes, const int *reps,
                       int numPoints, cudaStream_t s, std::vector<int> &u, std::vector<int> &v,
                       std::vector<float> &h);
 int denseLinkageFromMatrix(float *distances, const int *initialSize, const int *initialId,
-                           int firstNewId, int m, int linkageId, double *deviceTree,
+                           int firstNewId, int m, int linkageId, double *hostTree,
                            cudaStream_t s);
 
 namespace {
