@@ -167,12 +167,12 @@ __global__ void rnnMerge(const float *__restrict__ cent, const int *__restrict__
 // 206 (5 measured before the size term of screen.cuh got its updates).
 constexpr int kListK = 7;
 
-// With this many clusters or fewer every round searches all of them: the full
-// pass is then cheaper than the launches that would spare part of it (200,000 x
-// 32: a round at 4,000 clusters takes 0.2 ms with lists and 0.5 without, below
-// 800 about 0.15 either way; 3,916 x 8 in all, mostly such rounds: 10.1 ms with
-// lists throughout, 9.35 without).
-constexpr int kSearchAllBelow = 1024;
+// With this many clusters or fewer every round searches all of them for their
+// nearest alone: the full pass is then cheaper than the launches that would
+// spare part of it (passes of 200,000 x 32: a round at 4,000 clusters takes 0.2
+// ms with lists and 0.5 without, below 800 about 0.15 either way; 3,916 x 8 in
+// all, mostly such rounds: 10.1 ms with lists throughout, 9.35 without).
+constexpr int kSearchAllBelow = 2048;
 
 // The lists of all clusters, entry-major ([entry][slot], `stride` slots):
 // partners by representative and their exact weights, lightest first by (weight,
@@ -547,6 +547,7 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
     p.nodeHigh = index.nodeHigh.get();
     p.nodeMinValue = index.nodeMinValue.get();
     p.prune = prune;
+    p.nearest = nearest.get();
     p.k = kListK;
     p.knnParts = parts.get();
     p.tilesComputed = tiles.get();
@@ -555,7 +556,8 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
     p.screenAudit = screenAuditWords();
     WardWeight w;
     w.value = sizeF[cur].get();
-    if (rounds > 0 && m > kSearchAllBelow) {
+    const bool listed = m > kSearchAllBelow;
+    if (rounds > 0 && listed) {
       bool ordered = false;
       CUHC_TRY(st, index.selectRows(searchFlag.get(), nullptr, sizeF[cur].get(), &ordered));
       p.rowPos = index.rowPos.get();
@@ -569,7 +571,13 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
     }
     {
       PassTimer timer(screened ? kTimerScreenPass : kTimerNearestPass, s);
-      if (screened)
+      if (screened && !listed)
+        CUHC_TRY(st, (launchScreen<SqEuclideanMetric, WardWeight, false>(
+                         p, SqEuclideanMetric{}, w, index.kc, s)));
+      else if (!listed)
+        CUHC_TRY(st, (launchPass<SqEuclideanMetric, WardWeight, false>(p, SqEuclideanMetric{}, w,
+                                                                       index.kc, s)));
+      else if (screened)
         CUHC_TRY(st, (launchScreen<SqEuclideanMetric, WardWeight, true>(
                          p, SqEuclideanMetric{}, w, index.kc, s)));
       else
@@ -582,11 +590,12 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
         tilesSoFar = now;
       }
     }
-    collectLists<<<index.numTiles, kTile, 0, s>>>(parts.get(), p.rowTiles, p.rowPos,
-                                                  index.numTiles, index.numTiles, m,
-                                                  p.radius, listsOf(cur), rounding,
-                                                  nearest.get());
-    noteLaunch();
+    if (listed) {
+      collectLists<<<index.numTiles, kTile, 0, s>>>(parts.get(), p.rowTiles, p.rowPos,
+                                                    index.numTiles, index.numTiles, m, p.radius,
+                                                    listsOf(cur), rounding, nearest.get());
+      noteLaunch();
+    }
     rnnPartners<<<blocks(m), 256, 0, s>>>(nearest.get(), slotOfRep.get(), rep[cur].get(), m,
                                           partner.get(), survive.get());
     noteLaunch();
@@ -598,7 +607,7 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
         cent[nxt].get(), size[nxt].get(), sizeF[nxt].get(), rep[nxt].get(), slotOfRep.get(),
         changed.get(), mergeWeight.get(), nearest.get(), mergeU.get(), mergeV.get(), mergeH.get(), counter.get(), n - 1);
     noteLaunch();
-    if (m > kSearchAllBelow) {
+    if (listed) {
       updateLists<<<blocks(m, 128), 128, 0, s>>>(
           listsOf(cur), listsOf(nxt), partner.get(), mergeWeight.get(), newIndex.get(),
           rep[cur].get(), sizeF[cur].get(), m, slotOfRep.get(), cent[nxt].get(),

@@ -47,7 +47,15 @@ struct SpatialIndex {
   BvhTopology topo;
   DeviceBuffer<float> tiled;         // numTiles * numChunks * kc * 128
   DeviceBuffer<int> order, rank;     // position -> original, original -> position
-  DeviceBuffer<int> nodeLeft, nodeRight, nodeFirstTile, nodeTileCount, leafOfTile;
+  // The tree's index arrays, uploaded as one block (uploadTopology): children,
+  // first tile, tile count and parent per node, leaf per tile.
+  struct IntArray {
+    int *ptr = nullptr;
+    int *get() const { return ptr; }
+  };
+  DeviceBuffer<int> topology;
+  IntArray nodeLeft, nodeRight, nodeFirstTile, nodeTileCount, nodeParent, leafOfTile;
+  DeviceBuffer<int> nodeArrived; // children done, zero between the summary kernels
   DeviceBuffer<float> nodeLow, nodeHigh; // numNodes * d
   DeviceBuffer<float> nodeMinValue;      // numNodes
   DeviceBuffer<int> nodePure;            // numNodes: component if pure, else -1
@@ -87,6 +95,7 @@ struct SpatialIndex {
   // subtree (rootOfTile), so traversals never leave their instance.
   int buildBatch(const float *points, const std::vector<int> &sizes, int d,
                  cudaStream_t stream);
+  int uploadTopology();
   int buildCommon(const float *points, int positions, int d, bool spatial,
                   const std::vector<int> *hostOrder, cudaStream_t stream);
   // Re-tiles new point data already in position order (RNN centroids after a
