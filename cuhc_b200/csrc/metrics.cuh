@@ -186,8 +186,11 @@ struct MutualReachWeight {
   const float *value = nullptr; // core distances, by position
   float alpha = 1.0f;
   __device__ __forceinline__ float load(int i) const { return value[i]; }
+  // A NaN distance stays a NaN (fmaxf would drop it and leave the core
+  // distances, an edge where there is none).
   __device__ __forceinline__ float weight(float d, float ci, float cj) const {
-    return fmaxf(fmaxf(ci, cj), alpha == 1.0f ? d : d / alpha);
+    const float core = fmaxf(ci, cj), scaled = alpha == 1.0f ? d : d / alpha;
+    return core > scaled ? core : scaled;
   }
   __device__ __forceinline__ float distBound(float thr, float) const {
     if (!(thr < INFINITY))

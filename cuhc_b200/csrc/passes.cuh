@@ -245,6 +245,13 @@ place:
     pos[i] = j;
 }
 
+// A distance as a list entry: at least +0 (cosine rounding can give -1e-8). A
+// NaN stays a NaN, which compares below nothing and so enters no list; clamped
+// to 0 it would be the nearest point of all.
+__device__ __forceinline__ float listValue(float distance) {
+  return distance <= 0.0f ? 0.0f : distance;
+}
+
 // Offers value v of position j to a row's k-NN list. Inserts it when it
 // beats the k-th value and keeps `tie` = "some point outside the list lies at
 // exactly the k-th value": an insertion evicts the old k-th, which ties the
@@ -329,7 +336,7 @@ __device__ __forceinline__ void knnEpilogue(const PassParams &p, const Metric &m
         const float v = kWeighted
                             ? w.weight(m.finalize(a), rowVal[r], cm.value[g.col(c)])
                         : colPos == rowPos ? 0.0f
-                                           : fmaxf(m.finalize(a), 0.0f);
+                                           : listValue(m.finalize(a));
         if (kWeighted)
           offerByIndex(list, listPos + rowInTile * k, k, v, colOrig[g.col(c)]);
         else

@@ -44,7 +44,9 @@ static __global__ void __launch_bounds__(kRadixThreads)
       const int c = base + tid;
       unsigned int bin = 0xffffffffu;
       if (c < n) {
-        const float v = c == self ? 0.0f : fmaxf(d[c], 0.0f);
+        // NaN counts as +inf, so that it is nobody's neighbour.
+        const float raw = c == self ? 0.0f : d[c];
+        const float v = raw < INFINITY ? fmaxf(raw, 0.0f) : INFINITY;
         const unsigned int key = __float_as_uint(v);
         if (pass == 0 || (key >> (shift + 8)) == prefix)
           bin = (key >> shift) & 255u;

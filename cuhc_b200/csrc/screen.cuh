@@ -1193,7 +1193,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                   }
                 }
               } else if (kKnn) {
-                const float value = J * kTile + jj == myPos ? 0.0f : fmaxf(m.finalize(acc), 0.0f);
+                const float value = J * kTile + jj == myPos ? 0.0f : listValue(m.finalize(acc));
                 // Offer to the row's list (the k-th value kept in a register):
                 // a value below the k-th enters, and the boundary-tie flag
                 // follows knnOffer (passes.cuh): an insertion evicts the old
