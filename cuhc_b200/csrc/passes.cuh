@@ -68,6 +68,14 @@ struct ColumnMeta {
   float *value;
 };
 
+// Whether a k-NN row is done: its list holds k points at distance 0 and another
+// one is known to tie them, so nothing can change its values or its tie flag.
+// (Identical points, 20,000 x 2: every row went on through all column tiles,
+// 5 ms more.)
+__device__ __forceinline__ bool knnRowDone(float kth, int tie) {
+  return kth == 0.0f && tie != 0;
+}
+
 // Threads 0..127 (one row each) refresh the row filters and the block
 // threshold; everyone must call it (it synchronizes).
 template <class Metric, class Weight, bool kKnn>
@@ -85,7 +93,9 @@ __device__ __forceinline__ void refreshThresholds(const PassParams &p, const Met
       thr = lists[tid * p.k + p.k - 1];
       if (valid && !std::is_same<Weight, PlainWeight>::value && p.radius)
         thr = fminf(thr, p.radius[pos]);
-      if (valid)
+      const bool done =
+          std::is_same<Weight, PlainWeight>::value && knnRowDone(thr, sh.rowTie[tid]);
+      if (valid && !done)
         filter = m.filterBound(w.distBound(thr, w.load(pos)));
     } else {
       const unsigned long long key = sh.rowBest[tid];

@@ -719,7 +719,9 @@ __global__ void __launch_bounds__(kThreads, 2)
       thr = listKeyValue(lists[myRow * p.k + p.k - 1]);
       if (kWeighted && mySearch && p.radius)
         thr = fminf(thr, p.radius[myPos]);
-      F = mySearch ? m.screenBound(kWeighted ? w.distBound(thr, myVal) : thr) : -INFINITY;
+      const bool done = !kWeighted && knnRowDone(thr, tie);
+      F = mySearch && !done ? m.screenBound(kWeighted ? w.distBound(thr, myVal) : thr)
+                            : -INFINITY;
     } else {
       thr = rowBest == kEmptyKey ? INFINITY : keyWeight(rowBest);
       if (compSlot) {
@@ -1211,6 +1213,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                   dirty = true;
                 } else if (value == rowKth) {
                   tie = 1;
+                  dirty |= knnRowDone(rowKth, tie);
                 }
               } else {
                 const float weight = w.weight(m.finalize(acc), myVal, useValue ? cVal[jj] : 0.0f);

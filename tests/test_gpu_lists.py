@@ -79,3 +79,16 @@ def test_nan_rows_stay_disconnected():
     X[17, 3] = float("nan")
     with pytest.raises(RuntimeError, match="finite"):
         C.linkage(X, "single")
+
+
+@pytest.mark.parametrize("n, copies", [(300, 300), (900, 10), (900, 9), (1600, 200)])
+@pytest.mark.parametrize("d, k", [(3, 9), (40, 1), (40, 12)])
+def test_rows_done_early(screen, n, copies, d, k):
+    """Lists of nothing but equal points, with a tie outside the list or not."""
+    X = np.repeat(normal(n // copies, d, seed=d), copies, axis=0)
+    X = np.random.default_rng(n).permutation(X)
+    np.testing.assert_array_equal(C.linkage(X, "single"), O.single_linkage(X))
+    Z, core = hdbscan_tree(X, k)
+    Z_ref, core_ref = O.hdbscan_tree(X, k)
+    np.testing.assert_array_equal(core, core_ref)
+    np.testing.assert_array_equal(Z, Z_ref)
