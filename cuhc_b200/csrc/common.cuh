@@ -2,6 +2,7 @@
 // keys, device buffers from the stream-ordered pool, bounded waits.
 #pragma once
 
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
 #include <cuda_runtime.h>
@@ -151,6 +152,28 @@ template <typename T> struct DeviceBuffer {
   T *get() const { return ptr; }
   size_t bytes() const { return count * sizeof(T); }
 };
+
+// Lets `kernel` be launched with `bytes` of dynamic shared memory. The limit is
+// an attribute of the function that all threads of the process share. It is set
+// to the most that the device allows and never to less: set to each launch's own
+// size, a smaller call in another thread lowered it between a larger call's
+// attribute and its launch, which then failed.
+template <class Kernel> int allowDynamicShared(Kernel kernel, size_t bytes) {
+  cudaFuncAttributes attributes;
+  int device = 0, perBlock = 0;
+  StatusChain st;
+  CUHC_TRY(st, cudaFuncGetAttributes(&attributes, kernel));
+  CUHC_TRY(st, cudaGetDevice(&device));
+  CUHC_TRY(st, cudaDeviceGetAttribute(&perBlock, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+  if (!st.ok())
+    return st.code;
+  const int most = perBlock - (int)attributes.sharedSizeBytes;
+  if (bytes > (size_t)std::max(most, 0))
+    return (int)cudaErrorInvalidValue;
+  if (attributes.maxDynamicSharedSizeBytes < most)
+    CUHC_TRY(st, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+  return st.code;
+}
 
 // Iteration limit for every spin-wait in this library's kernels. A wait that
 // runs out records kErrorTimeout in the kernel's error word and returns.

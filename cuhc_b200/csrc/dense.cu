@@ -381,8 +381,7 @@ int denseLinkageFromMatrix(float *distances, const int *initialSize, const int *
     CUHC_TRY(st, spill.allocate(own * blocks, s));
     shared -= own * sizeof(int);
   }
-  CUHC_TRY(st, cudaFuncSetAttribute(denseMerges, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)shared));
+  CUHC_TRY(st, allowDynamicShared(denseMerges, shared));
   cudaLaunchConfig_t config{};
   config.gridDim = dim3(blocks);
   config.blockDim = dim3(kMergeThreads);

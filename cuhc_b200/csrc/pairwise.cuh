@@ -147,10 +147,9 @@ int launchPairwise(const float *tiledA, const float *tiledB, int nA, int nB, int
   const size_t dyn = (numChunks > 1 ? 4 : 2) * (size_t)kc * kTile * sizeof(float);
   const bool vector = nB % 4 == 0 && ((uintptr_t)out & 15) == 0;
   auto run = [&](auto kernel) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-    if (e != cudaSuccess)
-      return (int)e;
+    const int e = allowDynamicShared(kernel, dyn);
+    if (e != 0)
+      return e;
     kernel<<<grid, kThreads, dyn, s>>>(tiledA, tiledB, nA, nB, numChunks, vector, m, out);
     noteLaunch();
     return (int)cudaGetLastError();

@@ -794,10 +794,9 @@ int launchPass(const PassParams &p, const Metric &m, const Weight &w, int kc,
     return (int)cudaErrorMisalignedAddress;
   auto run = [&](auto kernel) {
     // Static (~18 KB) plus dynamic shared memory can pass the 48 KB default.
-    const cudaError_t e =
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dynBytes);
-    if (e != cudaSuccess)
-      return (int)e;
+    const int e = allowDynamicShared(kernel, dynBytes);
+    if (e != 0)
+      return e;
     kernel<<<p.numTiles, kThreads, dynBytes, stream>>>(p, m, w);
     noteLaunch();
     return (int)cudaGetLastError();

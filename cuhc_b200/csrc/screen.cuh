@@ -1444,10 +1444,9 @@ int launchScreen(const PassParams &p, const Metric &m, const Weight &w, int kc,
         misaligned(w.value) || misaligned(p.packedMeta))
       return (int)cudaErrorMisalignedAddress;
     auto run = [&](auto kernel) {
-      const cudaError_t e =
-          cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dynBytes);
-      if (e != cudaSuccess)
-        return (int)e;
+      const int e = allowDynamicShared(kernel, dynBytes);
+      if (e != 0)
+        return e;
       kernel<<<p.numTiles, kThreads, dynBytes, stream>>>(p, m, w, margin, stages, lead);
       noteLaunch();
       return (int)cudaGetLastError();
