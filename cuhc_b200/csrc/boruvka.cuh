@@ -872,6 +872,10 @@ float timeKnnSample(SpatialIndex &index, const Metric &metric, int k, bool scree
   return status == 0 ? ms : INFINITY;
 }
 
+template <class Metric> bool listsFit(int d, int k) {
+  return listPassFits<Metric, PlainWeight>(d, k);
+}
+
 // Whether this index's passes can run screened (metric, width, shared
 // memory, data extent), ignoring the screen mode's "off".
 template <class Metric> bool screenable(SpatialIndex &index, int k) {

@@ -141,15 +141,19 @@ int singleLinkageMst(const float *devPoints, int n, int d, const Metric &m, doub
   // included): the later rounds then know most rows' answers, or that they
   // cannot matter, without a search.
   const int k = std::min(kSingleListK, n);
+  const bool keepLists = listsFit<Metric>(d, k);
   KnnListBuffers lists;
   DeviceBuffer<float> kth;
-  CUHC_TRY(st, lists.allocate(n, k, s));
-  CUHC_TRY(st, kth.allocate(paddedToTiles(n), s));
+  if (keepLists) {
+    CUHC_TRY(st, lists.allocate(n, k, s));
+    CUHC_TRY(st, kth.allocate(paddedToTiles(n), s));
+  }
   KnnLists knn = lists.lists(k);
-  CUHC_TRY(st, coreDistances<Metric>(index, m, k, prune, kth.get(), &stats, s, nullptr, &knn,
-                                     true));
+  if (keepLists)
+    CUHC_TRY(st, coreDistances<Metric>(index, m, k, prune, kth.get(), &stats, s, nullptr, &knn,
+                                       true));
   CUHC_TRY(st, (boruvkaMst<Metric, PlainWeight>(index, m, PlainWeight{}, prune, edges, &stats, s,
-                                                nullptr, &knn)));
+                                                nullptr, keepLists ? &knn : nullptr)));
   HostEdges sorted;
   CUHC_TRY(st, sortEdgesToPinned(edges, edges.count, s, sorted));
   if (st.ok() && sorted.count != n - 1)
@@ -290,9 +294,10 @@ int batchTrees(const float *devPoints, const std::vector<int> &sizes,
     return st.code;
   // Lists for the rounds, as single calls keep them: of the largest rank, and
   // at least of the length single linkage keeps.
-  const bool keepLists = maxK <= kMaxKeptListK;
+  const bool keepLists =
+      maxK <= kMaxKeptListK && listsFit<Metric>(d, std::max(maxK, kSingleListK));
   const int listK = keepLists ? std::max(maxK, kSingleListK) : maxK;
-  ScreenOverride screen(tuneScreen(index, m, metricId, listK, core.get(), s));
+  ScreenOverride screen(tuneScreen(index, m, metricId, std::max(listK, 1), core.get(), s));
   CUHC_TRY(st, cudaMemsetAsync(core.get(), 0, core.bytes(), s));
   PassStats stats;
   KnnListBuffers lists;
@@ -301,8 +306,9 @@ int batchTrees(const float *devPoints, const std::vector<int> &sizes,
   KnnLists knn = lists.lists(listK);
   // Mutual reachability with core 0 is the plain distance (keys clamp at 0),
   // so single-linkage instances (rank 0) share the solve with HDBSCAN ones.
-  CUHC_TRY(st, coreDistances<Metric>(index, m, listK, true, core.get(), &stats, s, rank.get(),
-                                     keepLists ? &knn : nullptr));
+  if (listK > 0)
+    CUHC_TRY(st, coreDistances<Metric>(index, m, listK, true, core.get(), &stats, s, rank.get(),
+                                       keepLists ? &knn : nullptr));
   CUHC_TRY(st, index.updateMinValues(core.get()));
   MutualReachWeight weight;
   weight.value = core.get();

@@ -40,6 +40,7 @@ int pairwiseDistances(const float *A, int nA, const float *B, int nB, int d, con
   template int cuhc::coreDistances<M>(cuhc::SpatialIndex &, const M &, int, bool, float *,         \
                                       cuhc::PassStats *, cudaStream_t, const int *,                \
                                       cuhc::KnnLists *, bool);                                     \
+  template bool cuhc::listsFit<M>(int, int);                                                       \
   template bool cuhc::screenable<M>(cuhc::SpatialIndex &, int);                                    \
   template float cuhc::timeKnnSample<M>(cuhc::SpatialIndex &, const M &, int, bool, int, float *,  \
                                         cudaStream_t);                                             \

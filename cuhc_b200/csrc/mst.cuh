@@ -107,15 +107,19 @@ int coreDistances(SpatialIndex &index, const Metric &metric, int k, bool prune, 
                   PassStats *stats, cudaStream_t stream, const int *coreRank = nullptr,
                   KnnLists *lists = nullptr, bool rounds = false);
 
-// The same core distances for any 1 <= k <= n by radix select over chunks of
-// the materialised distance matrix (radix.cuh). Bit-identical to
-// coreDistances.
+// Whether a k-NN pass over d features can keep lists of k entries (a block's
+// shared memory holds them beside its features).
+template <class Metric> bool listsFit(int d, int k);
+
 template <class Metric> bool screenable(SpatialIndex &index, int k);
 
 template <class Metric>
 float timeKnnSample(SpatialIndex &index, const Metric &metric, int k, bool screened,
                     int sampleTiles, float *core, cudaStream_t stream);
 
+// The same core distances for any 1 <= k <= n by radix select over chunks of
+// the materialised distance matrix (radix.cuh). Bit-identical to
+// coreDistances.
 template <class Metric>
 int coreDistancesRadix(SpatialIndex &index, const Metric &metric, int k, float *core,
                        cudaStream_t stream);

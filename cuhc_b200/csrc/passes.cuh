@@ -778,29 +778,8 @@ __global__ void __launch_bounds__(kThreads, 2) passKernel(PassParams p, Metric m
   }
 }
 
-// Host launcher. KC follows the point layout (chunkWidthFor(d)).
-template <class Metric, class Weight, bool kKnn>
-int launchPass(const PassParams &p, const Metric &m, const Weight &w, int kc,
-               cudaStream_t stream) {
-  constexpr bool kWeighted = kKnn && !std::is_same<Weight, PlainWeight>::value;
-  const size_t listEntries = kKnn ? (size_t)kTile * p.k * (p.knnPos || kWeighted ? 2 : 1) : 0;
-  const size_t dynBytes = (size_t)3 * kc * kTile * sizeof(float) + 6 * kTile * sizeof(int) +
-                          (2 * (size_t)p.d + listEntries) * sizeof(float);
-  // Bulk copies need 16-byte aligned sources (pool allocations are 256-byte
-  // aligned; refuse anything else rather than fault).
-  auto misaligned = [](const void *ptr) { return ((uintptr_t)ptr & 15) != 0; };
-  if (misaligned(p.tiled) || misaligned(p.order) || misaligned(p.component) ||
-      misaligned(w.value))
-    return (int)cudaErrorMisalignedAddress;
-  auto run = [&](auto kernel) {
-    // Static (~18 KB) plus dynamic shared memory can pass the 48 KB default.
-    const int e = allowDynamicShared(kernel, dynBytes);
-    if (e != 0)
-      return e;
-    kernel<<<p.numTiles, kThreads, dynBytes, stream>>>(p, m, w);
-    noteLaunch();
-    return (int)cudaGetLastError();
-  };
+// Calls run(kernel) with the pass kernel of a point layout (chunkWidthFor(d)).
+template <class Metric, class Weight, bool kKnn, class Run> int withPassKernel(int kc, Run run) {
   switch (kc) {
   case 4:
     return run(passKernel<Metric, Weight, 4, kKnn>);
@@ -811,6 +790,46 @@ int launchPass(const PassParams &p, const Metric &m, const Weight &w, int kc,
   default:
     return run(passKernel<Metric, Weight, 32, kKnn>);
   }
+}
+
+// Dynamic shared memory of a pass over d features with per-row lists of k
+// entries (0: nearest mode), values and indices (indexed) or values alone.
+inline size_t passDynamicBytes(int kc, int d, int k, bool indexed) {
+  const size_t listEntries = (size_t)kTile * k * (indexed ? 2 : 1);
+  return (size_t)3 * kc * kTile * sizeof(float) + 6 * kTile * sizeof(int) +
+         (2 * (size_t)d + listEntries) * sizeof(float);
+}
+
+// Whether a pass with indexed lists of k entries fits the block's shared
+// memory (it holds 8 bytes per feature; lists of 9 fit up to about 19,000).
+template <class Metric, class Weight> bool listPassFits(int d, int k) {
+  const int kc = chunkWidthFor(d);
+  return withPassKernel<Metric, Weight, true>(kc, [&](auto kernel) {
+           return allowDynamicShared(kernel, passDynamicBytes(kc, d, k, true));
+         }) == 0;
+}
+
+// Host launcher. KC follows the point layout (chunkWidthFor(d)).
+template <class Metric, class Weight, bool kKnn>
+int launchPass(const PassParams &p, const Metric &m, const Weight &w, int kc,
+               cudaStream_t stream) {
+  constexpr bool kWeighted = kKnn && !std::is_same<Weight, PlainWeight>::value;
+  const size_t dynBytes = passDynamicBytes(kc, p.d, kKnn ? p.k : 0, p.knnPos || kWeighted);
+  // Bulk copies need 16-byte aligned sources (pool allocations are 256-byte
+  // aligned; refuse anything else rather than fault).
+  auto misaligned = [](const void *ptr) { return ((uintptr_t)ptr & 15) != 0; };
+  if (misaligned(p.tiled) || misaligned(p.order) || misaligned(p.component) ||
+      misaligned(w.value))
+    return (int)cudaErrorMisalignedAddress;
+  return withPassKernel<Metric, Weight, kKnn>(kc, [&](auto kernel) {
+    // Static (~18 KB) plus dynamic shared memory can pass the 48 KB default.
+    const int e = allowDynamicShared(kernel, dynBytes);
+    if (e != 0)
+      return e;
+    kernel<<<p.numTiles, kThreads, dynBytes, stream>>>(p, m, w);
+    noteLaunch();
+    return (int)cudaGetLastError();
+  });
 }
 
 } // namespace cuhc

@@ -518,6 +518,7 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
   // every round.
   const bool screened =
       st.ok() && useScreen<SqEuclideanMetric>(d, kListK) && index.extentsWithin(kScreenMaxExtent);
+  const bool canList = screened || listPassFits<SqEuclideanMetric, WardWeight>(d, kListK);
   std::vector<int> roundEnd;
   int m = n, merged = 0, cur = 0, rounds = 0;
   enum { kNone, kDense, kChain } tail = kNone;
@@ -556,7 +557,7 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
     p.screenAudit = screenAuditWords();
     WardWeight w;
     w.value = sizeF[cur].get();
-    const bool listed = m > kSearchAllBelow;
+    const bool listed = canList && m > kSearchAllBelow;
     if (rounds > 0 && listed) {
       bool ordered = false;
       CUHC_TRY(st, index.selectRows(searchFlag.get(), nullptr, sizeF[cur].get(), &ordered));
