@@ -61,6 +61,8 @@ lib.cuhc_screen_counters.restype = _int
 lib.cuhc_screen_counters.argtypes = [ctypes.POINTER(ctypes.c_uint64), _int]
 lib.cuhc_set_screen.restype = _int
 lib.cuhc_set_screen.argtypes = [_int]
+lib.cuhc_set_optional_memory.restype = _int
+lib.cuhc_set_optional_memory.argtypes = [ctypes.c_uint64]
 lib.cuhc_launch_count.restype = ctypes.c_uint64
 lib.cuhc_launch_count.argtypes = []
 lib.cuhc_set_timing.restype = _int
@@ -113,6 +115,12 @@ def set_screen(mode):
     and sqeuclidean up to 32 features), "on" or "off". Results are identical
     in every mode; only the time changes."""
     check(lib.cuhc_set_screen(SCREEN_MODES[mode]))
+
+
+def set_optional_memory(limit=None):
+    """Test hook: the largest device array (bytes) allocated only to save time;
+    calls go on without larger ones, to the same results. None: no limit."""
+    check(lib.cuhc_set_optional_memory(2 ** 64 - 1 if limit is None else limit))
 
 
 SCREEN_COUNTERS = ("rechecks", "slow_rows", "indicator_tiles", "masked_tiles", "prefiltered")

@@ -500,7 +500,8 @@ int boruvkaMst(SpatialIndex &index, const Metric &metric, const Weight &weight, 
   // (batch, 8 features) 2.5 / 3.4; 0.48 (500,000 x 16) 61.7 / 58.4; 0.25
   // (100,000 x 8, HDBSCAN) 1.02 / 1.22; 0.08 (1,000,000 x 8, HDBSCAN) 15.1 /
   // 12.9; 0.04 (batch, 2 features) 3.1 / 9.6.
-  const bool packRows = lists.pos && lists.tilesSearched > 0.5 * index.fullTilePairs();
+  const bool packRows = lists.pos && lists.tilesSearched > 0.5 * index.fullTilePairs() &&
+                        index.reserveRows(st);
   who.everyone = logRows; // training rows want every row's answer, every round
   DeviceBuffer<float> features, prediction, radius, targets;
   DeviceBuffer<int> compSize;

@@ -71,6 +71,9 @@ void setScreenShape(ScreenShape shape) {
   }
 }
 
+std::atomic<size_t> gOptionalMemory{~size_t(0)};
+size_t optionalMemoryLimit() { return gOptionalMemory.load(); }
+
 int pairwiseIntoMatrix(const float *points, int n, int d, int metricId, float p, float *out,
                        cudaStream_t s) {
   return withMetric(metricId, p, [&](auto m) {
@@ -141,13 +144,12 @@ int singleLinkageMst(const float *devPoints, int n, int d, const Metric &m, doub
   // included): the later rounds then know most rows' answers, or that they
   // cannot matter, without a search.
   const int k = std::min(kSingleListK, n);
-  const bool keepLists = listsFit<Metric>(d, k);
   KnnListBuffers lists;
   DeviceBuffer<float> kth;
-  if (keepLists) {
-    CUHC_TRY(st, lists.allocate(n, k, s));
-    CUHC_TRY(st, kth.allocate(paddedToTiles(n), s));
-  }
+  const bool keepLists = listsFit<Metric>(d, k) && lists.allocate(st, n, k, s) &&
+                         allocateOptional(st, kth, paddedToTiles(n), s);
+  if (!keepLists)
+    lists.release();
   KnnLists knn = lists.lists(k);
   if (keepLists)
     CUHC_TRY(st, coreDistances<Metric>(index, m, k, prune, kth.get(), &stats, s, nullptr, &knn,
@@ -179,10 +181,9 @@ int hdbscanTree(const float *devPoints, int n, int d, const Metric &m, int minSa
   // alpha 1 only (a list edge's weight then needs no distance) and lists
   // that fit shared memory twice over.
   const bool radix = coreMethod == kCoreRadix || minSamples > kMaxListK;
-  const bool keepLists = !radix && alpha == 1.0f && minSamples <= kMaxKeptListK && n > 1;
   KnnListBuffers lists;
-  if (keepLists)
-    CUHC_TRY(st, lists.allocate(n, minSamples, s));
+  const bool keepLists = !radix && alpha == 1.0f && minSamples <= kMaxKeptListK && n > 1 &&
+                         lists.allocate(st, n, minSamples, s);
   KnnLists knn = lists.lists(minSamples);
   // Radix select when asked for, or when the per-row lists would not fit
   // shared memory (the reference's Auto picks radix above k = 64).
@@ -294,15 +295,14 @@ int batchTrees(const float *devPoints, const std::vector<int> &sizes,
     return st.code;
   // Lists for the rounds, as single calls keep them: of the largest rank, and
   // at least of the length single linkage keeps.
-  const bool keepLists =
-      maxK <= kMaxKeptListK && listsFit<Metric>(d, std::max(maxK, kSingleListK));
-  const int listK = keepLists ? std::max(maxK, kSingleListK) : maxK;
+  const int keptK = std::max(maxK, kSingleListK);
+  KnnListBuffers lists;
+  const bool keepLists = maxK <= kMaxKeptListK && listsFit<Metric>(d, keptK) &&
+                         lists.allocate(st, positions, keptK, s);
+  const int listK = keepLists ? keptK : maxK;
   ScreenOverride screen(tuneScreen(index, m, metricId, std::max(listK, 1), core.get(), s));
   CUHC_TRY(st, cudaMemsetAsync(core.get(), 0, core.bytes(), s));
   PassStats stats;
-  KnnListBuffers lists;
-  if (keepLists)
-    CUHC_TRY(st, lists.allocate(positions, listK, s));
   KnnLists knn = lists.lists(listK);
   // Mutual reachability with core 0 is the plain distance (keys clamp at 0),
   // so single-linkage instances (rank 0) share the solve with HDBSCAN ones.
@@ -628,6 +628,13 @@ int cuhc_set_pruning(int mode) {
   if (mode < kPruneAuto || mode > kPruneNever)
     return kErrorInvalidAlgorithm;
   gPruneMode.store(mode);
+  return 0;
+}
+
+// Largest array allocated only to save time (test hook): larger ones count as
+// allocations that found no memory. ~0, the default, limits nothing.
+int cuhc_set_optional_memory(unsigned long long bytes) {
+  gOptionalMemory.store((size_t)bytes);
   return 0;
 }
 

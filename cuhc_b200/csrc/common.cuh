@@ -153,6 +153,25 @@ template <typename T> struct DeviceBuffer {
   size_t bytes() const { return count * sizeof(T); }
 };
 
+// The largest array that a call may allocate only to save time (k-NN lists,
+// packed copies of rows); any size unless a test lowers it.
+size_t optionalMemoryLimit();
+
+// Allocates an array that only saves time. Returns false, with no error, when
+// there is no memory for it: the caller goes on without.
+template <typename T>
+bool allocateOptional(StatusChain &st, DeviceBuffer<T> &buffer, size_t n, cudaStream_t s) {
+  if (!st.ok() || n * sizeof(T) > optionalMemoryLimit())
+    return false;
+  const int code = buffer.allocate(n, s);
+  if (code == (int)cudaErrorMemoryAllocation) {
+    cudaGetLastError(); // the launches' error checks must not see it
+    return false;
+  }
+  st(code);
+  return code == 0;
+}
+
 // Lets `kernel` be launched with `bytes` of dynamic shared memory. The limit is
 // an attribute of the function that all threads of the process share. It is set
 // to the most that the device allows and never to less: set to each launch's own

@@ -76,12 +76,19 @@ struct KnnLists {
 struct KnnListBuffers {
   DeviceBuffer<int> pos, tie;
   DeviceBuffer<float> val;
-  int allocate(int n, int k, cudaStream_t s) {
-    StatusChain st;
-    CUHC_TRY(st, pos.allocate(paddedToTiles(n) * k, s));
-    CUHC_TRY(st, val.allocate(paddedToTiles(n) * k, s));
-    CUHC_TRY(st, tie.allocate(n, s));
-    return st.code;
+  // False when there is no memory for them (no error): go on without lists.
+  bool allocate(StatusChain &st, int n, int k, cudaStream_t s) {
+    const bool ok = allocateOptional(st, pos, paddedToTiles(n) * k, s) &&
+                    allocateOptional(st, val, paddedToTiles(n) * k, s) &&
+                    allocateOptional(st, tie, n, s);
+    if (!ok)
+      release();
+    return ok;
+  }
+  void release() {
+    pos.release();
+    val.release();
+    tie.release();
   }
   KnnLists lists(int k) const { return KnnLists{pos.get(), val.get(), tie.get(), k}; }
 };

@@ -141,10 +141,12 @@ __global__ void rnnMerge(const float *__restrict__ cent, const int *__restrict__
     nextSizeF[to] = (float)merged;
     nextRep[to] = rep[i];
     slotOfRep[rep[i]] = to;
-    nextChanged[to] = j >= 0;
+    if (nextChanged)
+      nextChanged[to] = j >= 0;
     if (j >= 0) {
       slotOfRep[rep[j]] = to; // where the lists that name j find it now
-      nextMergeWeight[to] = keyWeight(nearest[i]);
+      if (nextMergeWeight)
+        nextMergeWeight[to] = keyWeight(nearest[i]);
       const float *a = cent + (size_t)i * d, *b = cent + (size_t)j * d;
       float squared = 0.0f;
       for (int k = 0; k < d; ++k) {
@@ -458,15 +460,7 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
     CUHC_TRY(st, sizeF[b].allocate(paddedToTiles(n), s));
     CUHC_TRY(st, size[b].allocate(n, s));
     CUHC_TRY(st, rep[b].allocate(paddedToTiles(n), s));
-    CUHC_TRY(st, listRep[b].allocate((size_t)n * kListK, s));
-    CUHC_TRY(st, listWeight[b].allocate((size_t)n * kListK, s));
-    CUHC_TRY(st, rootBound[b].allocate(n, s));
   }
-  CUHC_TRY(st, cap.allocate(n, s));
-  CUHC_TRY(st, mergeWeight.allocate(n, s));
-  CUHC_TRY(st, changed.allocate(n, s));
-  CUHC_TRY(st, searchFlag.allocate(n, s));
-  CUHC_TRY(st, parts.allocate(paddedToTiles(n) * kListK, s));
   CUHC_TRY(st, slotOfRep.allocate(n, s));
   CUHC_TRY(st, partner.allocate(n, s));
   CUHC_TRY(st, survive.allocate(n, s));
@@ -518,7 +512,26 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
   // every round.
   const bool screened =
       st.ok() && useScreen<SqEuclideanMetric>(d, kListK) && index.extentsWithin(kScreenMaxExtent);
-  const bool canList = screened || listPassFits<SqEuclideanMetric, WardWeight>(d, kListK);
+  // Lists, where there is room for them.
+  bool canList = n > kSearchAllBelow &&
+                 (screened || listPassFits<SqEuclideanMetric, WardWeight>(d, kListK));
+  for (int b = 0; b < 2; ++b)
+    canList = canList && allocateOptional(st, listRep[b], (size_t)n * kListK, s) &&
+              allocateOptional(st, listWeight[b], (size_t)n * kListK, s) &&
+              allocateOptional(st, rootBound[b], n, s);
+  canList = canList && allocateOptional(st, cap, n, s) &&
+            allocateOptional(st, mergeWeight, n, s) && allocateOptional(st, changed, n, s) &&
+            allocateOptional(st, searchFlag, n, s) &&
+            allocateOptional(st, parts, paddedToTiles(n) * kListK, s) && index.reserveRows(st);
+  if (!canList) {
+    for (int b = 0; b < 2; ++b) {
+      listRep[b].release();
+      listWeight[b].release();
+    }
+    changed.release();
+    mergeWeight.release();
+    parts.release();
+  }
   std::vector<int> roundEnd;
   int m = n, merged = 0, cur = 0, rounds = 0;
   enum { kNone, kDense, kChain } tail = kNone;
@@ -606,7 +619,8 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
     rnnMerge<<<blocks((long long)m * d), 256, 0, s>>>(
         cent[cur].get(), size[cur].get(), rep[cur].get(), partner.get(), newIndex.get(), m, d,
         cent[nxt].get(), size[nxt].get(), sizeF[nxt].get(), rep[nxt].get(), slotOfRep.get(),
-        changed.get(), mergeWeight.get(), nearest.get(), mergeU.get(), mergeV.get(), mergeH.get(), counter.get(), n - 1);
+        changed.get(), mergeWeight.get(), nearest.get(), mergeU.get(), mergeV.get(),
+        mergeH.get(), counter.get(), n - 1);
     noteLaunch();
     if (listed) {
       updateLists<<<blocks(m, 128), 128, 0, s>>>(

@@ -834,6 +834,42 @@ __global__ void __launch_bounds__(kTile)
 
 } // namespace
 
+// One block walks an instance 1024 positions a step (about a microsecond
+// each); a larger single instance goes through a device-wide select.
+bool SpatialIndex::selectsPerInstance() const { return numInstances > 1 || n <= 16384; }
+
+bool SpatialIndex::reserveRows(StatusChain &st) {
+  const bool ok = allocateOptional(st, rowTiled, (size_t)numTiles * tileFloats(), stream) &&
+                  allocateOptional(st, rowPos, (size_t)numTiles * kTile, stream) &&
+                  allocateOptional(st, rowPure, numTiles, stream) &&
+                  allocateOptional(st, rowBoxLow, (size_t)numTiles * d, stream) &&
+                  allocateOptional(st, rowBoxHigh, (size_t)numTiles * d, stream) &&
+                  allocateOptional(st, rowMinValue, numTiles, stream);
+  if (!ok) {
+    rowTiled.release();
+    rowPos.release();
+    return false;
+  }
+  CUHC_TRY(st, rowCount.allocate(1, stream));
+  CUHC_TRY(st, rowTiles.allocate(1, stream));
+  if (!selectsPerInstance()) {
+    CUHC_TRY(st, cub::DeviceSelect::Flagged(nullptr, selectBytes,
+                                            thrust::counting_iterator<int>(0),
+                                            (const unsigned char *)nullptr, rowPos.get(),
+                                            rowCount.get(), n, stream));
+    CUHC_TRY(st, selectTemp.allocate(std::max<size_t>(selectBytes, 1), stream));
+  }
+  if (numInstances > 1) {
+    std::vector<int> first(instanceFirstTile);
+    first.push_back(numTiles);
+    CUHC_TRY(st, instanceTile.allocate(first.size(), stream));
+    CUHC_TRY(st, cudaMemcpyAsync(instanceTile.get(), first.data(), first.size() * sizeof(int),
+                                 cudaMemcpyHostToDevice, stream));
+    CUHC_TRY(st, cudaStreamSynchronize(stream));
+  }
+  return st.ok();
+}
+
 int SpatialIndex::selectRows(const unsigned char *flag, const int *component,
                              const float *values, bool *ordered) {
   StatusChain st;
@@ -842,36 +878,9 @@ int SpatialIndex::selectRows(const unsigned char *flag, const int *component,
   if (order)
     CUHC_TRY(st, allocateTileOrder());
   const int slots = numTiles * kTile;
-  // One block walks an instance 1024 positions a step (about a microsecond
-  // each); a larger single instance goes through a device-wide select.
-  const bool perInstance = numInstances > 1 || n <= 16384;
-  if (!rowPos.get()) {
-    CUHC_TRY(st, rowPos.allocate(slots, stream));
-    CUHC_TRY(st, rowPure.allocate(numTiles, stream));
-    CUHC_TRY(st, rowTiled.allocate((size_t)numTiles * tileFloats(), stream));
-    CUHC_TRY(st, rowBoxLow.allocate((size_t)numTiles * d, stream));
-    CUHC_TRY(st, rowBoxHigh.allocate((size_t)numTiles * d, stream));
-    CUHC_TRY(st, rowMinValue.allocate(numTiles, stream));
-    CUHC_TRY(st, rowCount.allocate(1, stream));
-    CUHC_TRY(st, rowTiles.allocate(1, stream));
-    if (!perInstance) {
-      CUHC_TRY(st, cub::DeviceSelect::Flagged(nullptr, selectBytes,
-                                              thrust::counting_iterator<int>(0), flag,
-                                              rowPos.get(), rowCount.get(), n, stream));
-      CUHC_TRY(st, selectTemp.allocate(std::max<size_t>(selectBytes, 1), stream));
-    }
-    if (numInstances > 1) {
-      std::vector<int> first(instanceFirstTile);
-      first.push_back(numTiles);
-      CUHC_TRY(st, instanceTile.allocate(first.size(), stream));
-      CUHC_TRY(st, cudaMemcpyAsync(instanceTile.get(), first.data(), first.size() * sizeof(int),
-                                   cudaMemcpyHostToDevice, stream));
-      CUHC_TRY(st, cudaStreamSynchronize(stream));
-    }
-  }
   if (!st.ok())
     return st.code;
-  if (perInstance) {
+  if (selectsPerInstance()) {
     selectInstanceRows<<<numInstances, 1024, 0, stream>>>(
         flag, numInstances > 1 ? instanceTile.get() : nullptr, numTiles, n, rowPos.get());
   } else {

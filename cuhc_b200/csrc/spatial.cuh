@@ -134,7 +134,11 @@ struct SpatialIndex {
   // batch or where it matters, tileOrder: heaviest first by the work of the
   // rows' own tiles in the last full pass, row tiles without rows last.
   // *ordered tells whether it is in use. Enqueued on the index stream with no
-  // host work (buffers are allocated on first use).
+  // host work, after reserveRows.
+  bool selectsPerInstance() const;
+  // The buffers of selectRows; false when there is no memory for them (no
+  // error: the caller searches the rows in place).
+  bool reserveRows(StatusChain &st);
   int selectRows(const unsigned char *flag, const int *componentByPosition,
                  const float *valuesByPosition, bool *ordered);
   int allocateTileOrder();

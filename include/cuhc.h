@@ -169,6 +169,12 @@ int cuhc_mlp_train(const float *x, const float *y, int count, int epochs, int ba
  * change; returns CUHC_ERROR_INVALID_ALGORITHM for other values. */
 int cuhc_set_screen(int mode);
 
+/* Test hook: the largest device array, in bytes, that a call may allocate only
+ * to save time (k-NN lists kept for the rounds, packed copies of rows); a larger
+ * one counts as an allocation that found no memory, and the call goes on
+ * without, to the same result. All ones (the default) limits nothing. */
+int cuhc_set_optional_memory(unsigned long long bytes);
+
 /* Cumulative counters since load: out[0] tiles computed, out[1] tiles in all
  * passes, out[2] passes, out[3] Borůvka rounds (first `count` of them). */
 int cuhc_pass_stats(unsigned long long *out, int count);
