@@ -43,6 +43,8 @@ CASES = {
     "packed": lambda: normal(5000, 32, seed=8),
     "packed, device-wide select": lambda: normal(16_500, 20, seed=9),
     "two chunks": lambda: normal(3000, 40, seed=10),
+    # More row tiles than start at once: large components sit rounds out in place.
+    "sitting out in place": lambda: blobs(38_100, 2, centers=3, noise=0.2, seed=12),
 }
 
 
