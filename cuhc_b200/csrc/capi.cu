@@ -49,6 +49,16 @@ constexpr int kMaxKeptListK = 64;
 // 500,000 x 16 anisotropic 146 / 138 / 145 / 155, 20,000 x 32 6.9 / 6.2 / 6.0
 // / 6.1 (packed rows, one block per row tile).
 constexpr int kSingleListK = 9;
+// Points from which single linkage keeps lists when its passes are plain and the
+// metric has a filter. The list pass then costs a few nearest passes (a row's
+// first tiles enter one value at a time), and a small call has no more than that
+// to save. Whole calls in ms, with lists and without: chebyshev 8 features blobs
+// 1,000 points 1.52 / 1.02, 4,000 2.40 / 2.06, 8,000 3.14 / 2.82, normal 1,000
+// 1.14 / 0.81, 4,000 2.09 / 2.09, 8,000 2.47 / 2.94; euclidean 48 features blobs
+// 2,000 3.02 / 2.58, 4,000 5.06 / 4.92, 8,000 7.39 / 7.96. Cosine has no filter,
+// so its nearest passes are the dear ones: 48 features normal 300 points 1.85 /
+// 2.78, blobs 1,000 7.5 / 8.0.
+constexpr int kPlainListsFrom = 4096;
 
 std::atomic<int> gPruneMode{kPruneAuto};
 std::mutex gStatsMutex;
@@ -146,7 +156,8 @@ int singleLinkageMst(const float *devPoints, int n, int d, const Metric &m, doub
   const int k = std::min(kSingleListK, n);
   KnnListBuffers lists;
   DeviceBuffer<float> kth;
-  const bool keepLists = listsFit<Metric>(d, k) && lists.allocate(st, n, k, s) &&
+  const bool pays = n >= kPlainListsFrom || !Metric::kHasFilter || useScreen<Metric>(d, k);
+  const bool keepLists = pays && listsFit<Metric>(d, k) && lists.allocate(st, n, k, s) &&
                          allocateOptional(st, kth, paddedToTiles(n), s);
   if (!keepLists)
     lists.release();

@@ -176,6 +176,13 @@ constexpr int kListK = 7;
 // all, mostly such rounds: 10.1 ms with lists throughout, 9.35 without).
 constexpr int kSearchAllBelow = 2048;
 
+// Points from which lists are kept when the passes are plain: their list pass
+// offers values one at a time, which the later rounds have to earn back. Whole
+// calls in ms, with lists and without: 48 features blobs 10,000 24 / 20, 20,000
+// 40 / 34, 30,000 52 / 48, 40,000 63 / 68; normal 10,000 32 / 30, 20,000 49 / 53,
+// 40,000 85 / 126; 100 features blobs 20,000 59 / 58, 30,000 82 / 99.
+constexpr int kPlainListsFrom = 30000;
+
 // The lists of all clusters, entry-major ([entry][slot], `stride` slots):
 // partners by representative and their exact weights, lightest first by (weight,
 // representative), -1 / +inf past the last; the square root of the bound b.
@@ -513,8 +520,9 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
   const bool screened =
       st.ok() && useScreen<SqEuclideanMetric>(d, kListK) && index.extentsWithin(kScreenMaxExtent);
   // Lists, where there is room for them.
-  bool canList = n > kSearchAllBelow &&
-                 (screened || listPassFits<SqEuclideanMetric, WardWeight>(d, kListK));
+  bool canList = screened ? n > kSearchAllBelow
+                          : n >= kPlainListsFrom &&
+                                listPassFits<SqEuclideanMetric, WardWeight>(d, kListK);
   for (int b = 0; b < 2; ++b)
     canList = canList && allocateOptional(st, listRep[b], (size_t)n * kListK, s) &&
               allocateOptional(st, listWeight[b], (size_t)n * kListK, s) &&

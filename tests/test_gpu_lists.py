@@ -43,6 +43,11 @@ CASES = {
     "packed": lambda: normal(5000, 32, seed=8),
     "packed, device-wide select": lambda: normal(16_500, 20, seed=9),
     "two chunks": lambda: normal(3000, 40, seed=10),
+    # Enough points for lists in plain passes.
+    "large grid": lambda: grid(65),
+    "many duplicates": lambda: np.repeat(blobs(250, 4, seed=13), 18, axis=0),
+    "long chain": lambda: np.cumsum(np.linspace(1, 2, 4200))[:, None].astype(np.float32),
+    "two chunks, packed": lambda: normal(4100, 40, seed=14),
     # More row tiles than start at once: large components sit rounds out in place.
     "sitting out in place": lambda: blobs(38_100, 2, centers=3, noise=0.2, seed=12),
 }

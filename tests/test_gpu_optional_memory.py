@@ -18,7 +18,7 @@ LIMITS = {"nothing": 0, "lists only": 24 * 128 * 9 * 4}
 
 CALLS = {
     "single": lambda: (C.linkage(normal(N, D, seed=1), "single"),),
-    "single, several chunks": lambda: (C.linkage(normal(N, 40, seed=1), "single"),),
+    "single, several chunks": lambda: (C.linkage(normal(N, 40, seed=1), "single", "cosine"),),
     "hdbscan": lambda: hdbscan_tree(normal(N, D, seed=2), 9),
     "ward": lambda: (C.linkage(normal(N, D, seed=3), "ward"),),
     "batch": lambda: [a for pair in C.batched_trees(

@@ -15,9 +15,11 @@ pytestmark = pytest.mark.gpu
 WIDE = 19_800
 
 
-def test_single_linkage():
+@pytest.mark.parametrize("metric", ["euclidean", "cosine"])
+def test_single_linkage(metric):
     X = blobs(300, WIDE, seed=1)
-    np.testing.assert_array_equal(C.linkage(X, "single"), O.single_linkage(X))
+    np.testing.assert_array_equal(C.linkage(X, "single", metric=metric),
+                                  O.single_linkage(X, metric=metric))
 
 
 def test_batch():
