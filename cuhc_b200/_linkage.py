@@ -93,6 +93,18 @@ def _ward_rnn_with_options(X, min_progress, dense_below=0, allow_dense=True):
     return tree
 
 
+def _dense_with_options(X, method, metric="euclidean", p=2.0, resident_slots=-1):
+    """Test hook: the dense algorithm with the point count up to which one
+    resident cluster makes the merges (0: never)."""
+    X = as_points(X, "X")
+    n = X.shape[0]
+    tree = np.empty((max(n - 1, 0), 4), dtype=np.float64)
+    _lib.check(_lib.lib.cuhc_linkage_dense_with_options(
+        _lib.float_ptr(X), n, X.shape[1], METRIC_IDS[metric], float(p), LINKAGE_IDS[method],
+        int(resident_slots), _lib.double_ptr(tree)))
+    return tree
+
+
 def cut_tree(Z, num_merges):
     """Labels 0..k-1 of the leaves after the first num_merges merges of Z."""
     Z = np.asarray(Z)

@@ -499,6 +499,25 @@ int cuhc_ward_rnn_with_options(const float *hostPoints, int n, int d, float minP
   return st.code;
 }
 
+int cuhc_linkage_dense_with_options(const float *hostPoints, int n, int d, int metricId, float p,
+                                    int linkageId, int residentSlots, double *hostTree) {
+  const int invalid = validateLinkage(n, d, metricId, linkageId, kDense);
+  if (invalid)
+    return invalid;
+  if (n == 1)
+    return 0;
+  CallContext ctx;
+  StatusChain st;
+  st(ctx.status);
+  DeviceBuffer<float> points;
+  CUHC_TRY(st, points.allocate((size_t)n * d, ctx.stream));
+  CUHC_TRY(st, cudaMemcpyAsync(points.get(), hostPoints, points.bytes(), cudaMemcpyHostToDevice,
+                               ctx.stream));
+  CUHC_TRY(st, denseLinkage(points.get(), n, d, metricId, p, linkageId, hostTree, ctx.stream,
+                            residentSlots));
+  return st.code;
+}
+
 int cuhc_hdbscan_tree(const float *hostPoints, int n, int d, int metricId, float p,
                       int minSamples, float alpha, int coreMethod, double *hostTree,
                       float *hostCore) {

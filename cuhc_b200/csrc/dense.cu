@@ -9,15 +9,15 @@
 // was a or b and got farther. The reference does the same three steps per
 // merge (linkage.cuh:86-268) with the same tie rules and formulas.
 //
-// B200 shape: a merge is a chain of short dependent steps, so all of them run
-// in one thread-block cluster that stays resident for the whole tree. The slots
-// are dealt out over its blocks, whose shared memory holds their nearest
-// neighbours and sizes; per merge the blocks exchange their minima through
-// distributed shared memory around one cluster barrier, and read and write the
-// matrix through L2. A merge is bound by that chain's latency (reduction,
-// barrier, two row reads, the rescans): 5 us at 300 and 1,000 points, 6.3 at
-// 3,001 and 20 at 16,000, where a captured graph of four kernels per merge, each
-// a launch and a pass through memory, took 13, 12, 11 and 25 us.
+// B200 shape: a merge is a chain of short dependent steps. Up to a few thousand
+// slots all merges run in one thread-block cluster that stays resident for the
+// whole tree: the slots are dealt out over its blocks, whose shared memory holds
+// their nearest neighbours and sizes; per merge the blocks exchange their minima
+// through distributed shared memory around one cluster barrier, and read and
+// write the matrix through L2. That is bound by the chain's latency (reduction,
+// barrier, two row reads, the rescans). With more slots a merge is a captured
+// graph of four kernels over the whole GPU (three launches' latency, and the
+// bandwidth of all SMs for the rescans). Both take the same merges, bit for bit.
 #include "profiling.cuh"
 #include "rnn.cuh"
 
@@ -42,9 +42,17 @@ constexpr int kRescanThreads = 256;
 // Blocks of the cluster (the portable limit) and their threads; a block takes
 // fewer than kMinSlots slots only when it is alone.
 constexpr int kClusterBlocks = 8, kMergeThreads = 512, kMinSlots = 128;
-// Dynamic shared memory a block of the cluster may take (227 KiB per block,
-// less its static arrays).
-constexpr size_t kDenseShared = 224 * 1024;
+// Slots up to which the cluster makes the merges. Its eight blocks lose to the
+// whole GPU where many rows lose their nearest slot per merge: some points are
+// many others' nearest, the more so the more features there are. Average linkage
+// of normal points in ms, cluster / whole GPU: 2 features 4,000 points 23 / 46,
+// 8,000 70 / 121, 20,000 337 / 507; 64 features 4,000 35 / 48, 6,000 73 / 83, 8,000
+// 121 / 125, 20,000 698 / 526; 300 features 4,000 47 / 49, 5,000 72 / 65, 20,000
+// 1,443 / 538; 1,000 features 3,072 34 / 37, 4,096 55 / 49. Ward of 400-fold
+// duplicates, 8 features: 6,000 75 / 85, 8,000 118 / 115.
+inline int residentSlotsFor(int d) { return d <= 64 ? 7168 : 3072; }
+// The wide form: threads of the reducing block, merges per captured graph.
+constexpr int kReduceThreads = 1024, kStepsPerGraph = 64;
 enum LinkageKind : int { kSingleL = 0, kCompleteL = 1, kAverageL = 2, kWardL = 3 };
 
 // One merge: slots a < b at `distance` into a cluster of `size` points.
@@ -78,45 +86,52 @@ __device__ __forceinline__ bool lessLoc(float da, int ia, float db, int ib) {
   return da < db || (da == db && ia < ib);
 }
 
-// Nearest other slot of every row.
-__global__ void __launch_bounds__(kRescanThreads)
-    denseNearest(float *__restrict__ dist, int n, float *__restrict__ nearDist,
-                 int *__restrict__ nearSlot) {
+// The nearest other slot of a row, by one block of kRescanThreads.
+__device__ __forceinline__ void nearestOfRow(const float *__restrict__ r, int n, int row,
+                                             float *nearDist, int *nearSlot) {
   __shared__ float wd[kRescanThreads / 32];
   __shared__ int ws[kRescanThreads / 32];
-  for (int row = blockIdx.x; row < n; row += gridDim.x) {
-    const float *r = dist + (size_t)row * n;
-    float best = INFINITY;
-    int slot = 0x7fffffff;
-    for (int c = threadIdx.x; c < n; c += kRescanThreads)
-      if (c != row && lessLoc(r[c], c, best, slot)) {
-        best = r[c];
-        slot = c;
-      }
-    for (int off = 16; off > 0; off /= 2) {
-      const float od = __shfl_xor_sync(0xffffffffu, best, off);
-      const int os = __shfl_xor_sync(0xffffffffu, slot, off);
-      if (lessLoc(od, os, best, slot)) {
-        best = od;
-        slot = os;
-      }
+  float best = INFINITY;
+  int slot = 0x7fffffff;
+#pragma unroll 4
+  for (int c = threadIdx.x; c < n; c += kRescanThreads) {
+    const float x = r[c]; // loaded whatever c is, so that the loads overlap
+    if (c != row && lessLoc(x, c, best, slot)) {
+      best = x;
+      slot = c;
     }
-    if ((threadIdx.x & 31) == 0) {
-      wd[threadIdx.x >> 5] = best;
-      ws[threadIdx.x >> 5] = slot;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int w = 1; w < kRescanThreads / 32; ++w)
-        if (lessLoc(wd[w], ws[w], best, slot)) {
-          best = wd[w];
-          slot = ws[w];
-        }
-      nearDist[row] = best;
-      nearSlot[row] = slot;
-    }
-    __syncthreads();
   }
+  for (int off = 16; off > 0; off /= 2) {
+    const float od = __shfl_xor_sync(0xffffffffu, best, off);
+    const int os = __shfl_xor_sync(0xffffffffu, slot, off);
+    if (lessLoc(od, os, best, slot)) {
+      best = od;
+      slot = os;
+    }
+  }
+  if ((threadIdx.x & 31) == 0) {
+    wd[threadIdx.x >> 5] = best;
+    ws[threadIdx.x >> 5] = slot;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kRescanThreads / 32; ++w)
+      if (lessLoc(wd[w], ws[w], best, slot)) {
+        best = wd[w];
+        slot = ws[w];
+      }
+    *nearDist = best;
+    *nearSlot = slot;
+  }
+  __syncthreads();
+}
+
+// Nearest other slot of every row.
+__global__ void __launch_bounds__(kRescanThreads)
+    denseNearest(const float *__restrict__ dist, int n, float *__restrict__ nearDist,
+                 int *__restrict__ nearSlot) {
+  for (int row = blockIdx.x; row < n; row += gridDim.x)
+    nearestOfRow(dist + (size_t)row * n, n, row, &nearDist[row], &nearSlot[row]);
 }
 
 // (distance, slot) as a key whose unsigned order is lessLoc's (-0 as +0).
@@ -174,8 +189,7 @@ __device__ __forceinline__ unsigned long long scanRow(const float *__restrict__ 
 __global__ void __launch_bounds__(kMergeThreads)
     denseMerges(float *__restrict__ dist, int n, int perBlock, int linkage,
                 const float *__restrict__ nearDist0, const int *__restrict__ nearSlot0,
-                const int *__restrict__ initialSize, float *__restrict__ spill,
-                MergeRecord *__restrict__ merges, int *__restrict__ mergeCount) {
+                const int *__restrict__ initialSize, MergeRecord *__restrict__ merges, int *__restrict__ mergeCount) {
   extern __shared__ __align__(16) unsigned char dense_shared[];
   __shared__ MergeNote notes[2][kClusterBlocks];
   __shared__ unsigned long long warpBest[kMergeThreads / 32], warpRow[kMergeThreads / 32];
@@ -184,9 +198,7 @@ __global__ void __launch_bounds__(kMergeThreads)
   const int rank = (int)cluster.block_rank(), blocks = (int)cluster.num_blocks();
   int *size = reinterpret_cast<int *>(dense_shared);
   unsigned int *active = reinterpret_cast<unsigned int *>(size + perBlock);
-  // The block's own: in shared memory, or past its reach in `spill`.
-  float *nearDist = spill ? spill + (size_t)rank * 3 * perBlock
-                          : reinterpret_cast<float *>(active + (n + 31) / 32);
+  float *nearDist = reinterpret_cast<float *>(active + (n + 31) / 32);
   int *nearSlot = reinterpret_cast<int *>(nearDist + perBlock);
   int *lost = nearSlot + perBlock;
 
@@ -337,6 +349,113 @@ __global__ void __launch_bounds__(kMergeThreads)
   cluster.sync(); // no block's shared memory goes while another may read it
 }
 
+// ---- the wide form: a merge as four kernels ----
+
+struct WideState {
+  float *dist, *nearDist;
+  int *nearSlot, *size, *lost, *lostCount, *step;
+  unsigned char *active;
+  MergeRecord *merges;
+  int n, linkage;
+};
+
+__global__ void wideStart(WideState s, const int *__restrict__ initialSize) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= s.n)
+    return;
+  s.dist[(size_t)i * s.n + i] = INFINITY;
+  s.size[i] = initialSize ? initialSize[i] : 1;
+  s.active[i] = 1;
+  if (i == 0)
+    *s.lostCount = *s.step = 0;
+}
+
+// One block: the closest pair, its record, the bookkeeping of its slots. Without
+// a finite pair the step goes past the last merge, which ends the tree early.
+__global__ void __launch_bounds__(kReduceThreads) wideClosest(WideState s) {
+  const int step = *s.step, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (step >= s.n - 1)
+    return;
+  __shared__ unsigned long long warpBest[kReduceThreads / 32];
+  unsigned long long best = kEmptyKey;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < s.n; i += kReduceThreads) {
+    const float d = s.nearDist[i];
+    best = minKey(best, d < INFINITY ? locKey(d, i) : kEmptyKey);
+  }
+  best = warpMinKey(best);
+  if (lane == 0)
+    warpBest[warp] = best;
+  __syncthreads();
+  if (warp != 0)
+    return;
+  best = warpMinKey(warpBest[lane]);
+  if (lane != 0)
+    return;
+  if (best == kEmptyKey) {
+    *s.step = s.n;
+    return;
+  }
+  const int slot = (int)(uint32_t)best, other = s.nearSlot[slot];
+  const int a = min(slot, other), b = max(slot, other);
+  const int merged = s.size[a] + s.size[b];
+  s.merges[step] = MergeRecord{a, b, orderedFloat((uint32_t)(best >> 32)), merged};
+  s.size[a] = merged;
+  s.active[b] = 0;
+  s.nearDist[b] = INFINITY;
+  *s.lostCount = 0;
+}
+
+// One thread per slot k: its distance to the merged cluster, and its nearest
+// slot kept, taken or lost. Retired columns hold +inf.
+__global__ void wideMerge(WideState s) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x, step = *s.step;
+  if (k >= s.n || step >= s.n - 1 || !s.active[k])
+    return;
+  const MergeRecord merge = s.merges[step];
+  const int a = merge.a, b = merge.b, sizeB = s.size[b];
+  const size_t n = s.n;
+  if (k == a) {
+    s.dist[(size_t)a * n + b] = INFINITY;
+    s.lost[atomicAdd(s.lostCount, 1)] = a;
+    return;
+  }
+  const float nd =
+      (float)lanceWilliams(s.linkage, s.dist[(size_t)a * n + k], s.dist[(size_t)b * n + k],
+                           merge.distance, merge.size - sizeB, sizeB, s.size[k]);
+  s.dist[(size_t)a * n + k] = nd;
+  s.dist[(size_t)k * n + a] = nd;
+  s.dist[(size_t)k * n + b] = INFINITY;
+  const int near = s.nearSlot[k];
+  if (near == a || near == b) {
+    if (nd <= s.nearDist[k]) {
+      s.nearDist[k] = nd;
+      s.nearSlot[k] = a;
+    } else {
+      s.lost[atomicAdd(s.lostCount, 1)] = k;
+    }
+  } else if (nd < s.nearDist[k]) {
+    s.nearDist[k] = nd;
+    s.nearSlot[k] = a;
+  }
+}
+
+// The nearest slots of the rows that lost theirs, a block per row.
+__global__ void __launch_bounds__(kRescanThreads) wideRescan(WideState s) {
+  if (*s.step >= s.n - 1)
+    return;
+  const int count = *s.lostCount;
+  for (int item = blockIdx.x; item < count; item += gridDim.x) {
+    const int row = s.lost[item];
+    nearestOfRow(s.dist + (size_t)row * s.n, s.n, row, &s.nearDist[row], &s.nearSlot[row]);
+  }
+}
+
+__global__ void wideAdvance(WideState s) {
+  if (*s.step < s.n - 1)
+    ++*s.step;
+}
+
 __global__ void wardTransform(float *dist, const int *size, int m) {
   const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (e >= (long long)m * m)
@@ -348,9 +467,94 @@ __global__ void wardTransform(float *dist, const int *size, int m) {
 
 } // namespace
 
+namespace {
+
+// All merges by the resident cluster.
+int mergeResident(float *distances, int m, int linkageId, const float *nearDist,
+                  const int *nearSlot, const int *initialSize, MergeRecord *merges,
+                  int *mergeCount, cudaStream_t s) {
+  StatusChain st;
+  int blocks = 1;
+  while (blocks < kClusterBlocks && m > blocks * kMinSlots)
+    blocks *= 2;
+  const int perBlock = (m + blocks - 1) / blocks;
+  const size_t shared = ((size_t)4 * perBlock + (m + 31) / 32) * sizeof(int);
+  CUHC_TRY(st, allowDynamicShared(denseMerges, shared));
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(blocks);
+  config.blockDim = dim3(kMergeThreads);
+  config.dynamicSmemBytes = shared;
+  config.stream = s;
+  cudaLaunchAttribute attribute{};
+  attribute.id = cudaLaunchAttributeClusterDimension;
+  attribute.val.clusterDim.x = blocks;
+  attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  CUHC_TRY(st, cudaLaunchKernelEx(&config, denseMerges, distances, m, perBlock, linkageId,
+                                  nearDist, nearSlot, initialSize, merges, mergeCount));
+  noteLaunch();
+  return st.code;
+}
+
+// All merges by replays of a graph of kStepsPerGraph of them: the step counter
+// lives on the device, and surplus steps leave at once.
+int mergeWide(float *distances, int m, int linkageId, float *nearDist, int *nearSlot,
+              const int *initialSize, MergeRecord *merges, int *step, int sms, cudaStream_t s) {
+  StatusChain st;
+  DeviceBuffer<int> ints;
+  DeviceBuffer<unsigned char> active;
+  CUHC_TRY(st, ints.allocate((size_t)2 * m + 1, s));
+  CUHC_TRY(st, active.allocate(m, s));
+  if (!st.ok())
+    return st.code;
+  WideState state{};
+  state.dist = distances;
+  state.nearDist = nearDist;
+  state.nearSlot = nearSlot;
+  state.size = ints.get();
+  state.lost = ints.get() + m;
+  state.lostCount = ints.get() + 2 * (size_t)m;
+  state.step = step;
+  state.active = active.get();
+  state.merges = merges;
+  state.n = m;
+  state.linkage = linkageId;
+  const int perSlot = (m + 255) / 256;
+  wideStart<<<perSlot, 256, 0, s>>>(state, initialSize);
+  noteLaunch();
+  CUHC_TRY(st, cudaGetLastError());
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  CUHC_TRY(st, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+  if (st.ok()) {
+    for (int i = 0; i < kStepsPerGraph; ++i) {
+      wideClosest<<<1, kReduceThreads, 0, s>>>(state);
+      wideMerge<<<perSlot, 256, 0, s>>>(state);
+      wideRescan<<<4 * sms, kRescanThreads, 0, s>>>(state);
+      wideAdvance<<<1, 1, 0, s>>>(state);
+    }
+    CUHC_TRY(st, cudaStreamEndCapture(s, &graph));
+  }
+  CUHC_TRY(st, cudaGraphInstantiate(&exec, graph, 0));
+  const int replays = (m - 1 + kStepsPerGraph - 1) / kStepsPerGraph;
+  for (int r = 0; r < replays && st.ok(); ++r) {
+    CUHC_TRY(st, cudaGraphLaunch(exec, s));
+    noteLaunch(4 * kStepsPerGraph);
+  }
+  CUHC_TRY(st, cudaStreamSynchronize(s));
+  if (exec)
+    cudaGraphExecDestroy(exec);
+  if (graph)
+    cudaGraphDestroy(graph);
+  return st.code;
+}
+
+} // namespace
+
 int denseLinkageFromMatrix(float *distances, const int *initialSize, const int *initialId,
                            int firstNewId, int m, int linkageId, double *hostTree,
-                           cudaStream_t s) {
+                           cudaStream_t s, int residentSlots) {
   if (m < 2)
     return 0;
   StatusChain st;
@@ -370,33 +574,12 @@ int denseLinkageFromMatrix(float *distances, const int *initialSize, const int *
                                                                nearSlot.get());
   noteLaunch();
   CUHC_TRY(st, cudaGetLastError());
-  int blocks = 1;
-  while (blocks < kClusterBlocks && m > blocks * kMinSlots)
-    blocks *= 2;
-  const int perBlock = (m + blocks - 1) / blocks;
-  const size_t own = (size_t)3 * perBlock;
-  size_t shared = ((size_t)perBlock + (m + 31) / 32 + own) * sizeof(int);
-  DeviceBuffer<float> spill;
-  if (shared > kDenseShared) {
-    CUHC_TRY(st, spill.allocate(own * blocks, s));
-    shared -= own * sizeof(int);
-  }
-  CUHC_TRY(st, allowDynamicShared(denseMerges, shared));
-  cudaLaunchConfig_t config{};
-  config.gridDim = dim3(blocks);
-  config.blockDim = dim3(kMergeThreads);
-  config.dynamicSmemBytes = shared;
-  config.stream = s;
-  cudaLaunchAttribute attribute{};
-  attribute.id = cudaLaunchAttributeClusterDimension;
-  attribute.val.clusterDim.x = blocks;
-  attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
-  config.attrs = &attribute;
-  config.numAttrs = 1;
-  CUHC_TRY(st, cudaLaunchKernelEx(&config, denseMerges, distances, m, perBlock, linkageId,
-                                  (const float *)nearDist.get(), (const int *)nearSlot.get(),
-                                  initialSize, spill.get(), merges.get(), mergeCount.get()));
-  noteLaunch();
+  if (m <= residentSlots)
+    CUHC_TRY(st, mergeResident(distances, m, linkageId, nearDist.get(), nearSlot.get(),
+                               initialSize, merges.get(), mergeCount.get(), s));
+  else
+    CUHC_TRY(st, mergeWide(distances, m, linkageId, nearDist.get(), nearSlot.get(), initialSize,
+                           merges.get(), mergeCount.get(), sms, s));
   std::vector<MergeRecord> host(m - 1);
   std::vector<int> id(m);
   int count = 0;
@@ -427,14 +610,15 @@ int denseLinkageFromMatrix(float *distances, const int *initialSize, const int *
 }
 
 int denseLinkage(const float *devPoints, int n, int d, int metricId, float p, int linkageId,
-                 double *hostTree, cudaStream_t s) {
+                 double *hostTree, cudaStream_t s, int residentSlots) {
   if (n < 2)
     return 0;
   StatusChain st;
   DeviceBuffer<float> dist;
   CUHC_TRY(st, dist.allocate((size_t)n * n, s));
   CUHC_TRY(st, pairwiseIntoMatrix(devPoints, n, d, metricId, p, dist.get(), s));
-  CUHC_TRY(st, denseLinkageFromMatrix(dist.get(), nullptr, nullptr, n, n, linkageId, hostTree, s));
+  CUHC_TRY(st, denseLinkageFromMatrix(dist.get(), nullptr, nullptr, n, n, linkageId, hostTree, s,
+                                      residentSlots >= 0 ? residentSlots : residentSlotsFor(d)));
   return st.code;
 }
 
@@ -450,7 +634,7 @@ int denseOnWardMatrix(const float *centroids, const int *sizes, const int *reps,
   CUHC_TRY(st, cudaGetLastError());
   std::vector<double> host((size_t)(m - 1) * 4);
   CUHC_TRY(st, denseLinkageFromMatrix(dist.get(), sizes, reps, numPoints, m, kWardL, host.data(),
-                                      s));
+                                      s, residentSlotsFor(d)));
   if (!st.ok())
     return st.code;
   // Tree ids -> representative points: a new cluster is represented by the

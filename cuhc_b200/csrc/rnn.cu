@@ -51,7 +51,7 @@ int denseOnWardMatrix(const float *centroids, const int *sizes, const int *reps,
                       std::vector<float> &h);
 int denseLinkageFromMatrix(float *distances, const int *initialSize, const int *initialId,
                            int firstNewId, int m, int linkageId, double *hostTree,
-                           cudaStream_t s);
+                           cudaStream_t s, int residentSlots);
 
 namespace {
 

@@ -23,9 +23,10 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
 // Ward by the nearest-neighbour chain.
 int nnChainWard(const float *devPoints, int n, int d, double *hostTree, cudaStream_t stream);
 
-// Any linkage on the dense n x n float32 matrix (Lance-Williams updates).
+// Any linkage on the dense n x n float32 matrix (Lance-Williams updates), in one
+// resident cluster up to residentSlots points (-1: dense.cu's own line).
 int denseLinkage(const float *devPoints, int n, int d, int metricId, float p, int linkageId,
-                 double *hostTree, cudaStream_t stream);
+                 double *hostTree, cudaStream_t stream, int residentSlots = -1);
 
 // The pruning mode set by cuhc_set_pruning (0 auto, 1 always, 2 never).
 int currentPruneMode();

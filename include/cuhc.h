@@ -169,6 +169,14 @@ int cuhc_mlp_train(const float *x, const float *y, int count, int epochs, int ba
  * change; returns CUHC_ERROR_INVALID_ALGORITHM for other values. */
 int cuhc_set_screen(int mode);
 
+/* Test hook: cuhc_linkage's dense algorithm with the number of points up to which
+ * one resident thread-block cluster makes the merges (-1: the default); above it
+ * every merge uses the whole GPU. The tree is the same. A cluster that does not
+ * fit its shared memory (above about 100,000 points) is refused. */
+int cuhc_linkage_dense_with_options(const float *points, int numPoints, int numFeatures,
+                                    int metricId, float metricParam, int linkageId,
+                                    int residentSlots, double *tree);
+
 /* Test hook: the largest device array, in bytes, that a call may allocate only
  * to save time (k-NN lists kept for the rounds, packed copies of rows); a larger
  * one counts as an allocation that found no memory, and the call goes on

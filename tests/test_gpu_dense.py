@@ -2,13 +2,16 @@
 merge rules on the host: the closest pair by (distance, slot), Lance-Williams
 updates in double rounded to float32, the merged cluster in the lower slot, a
 cached nearest slot kept unless its cluster merged and got farther. Sizes around
-the cluster's splits (1, 2, 4, 8 blocks), long rows, ties everywhere, duplicates, negative cosine distances."""
+the cluster's splits (1, 2, 4, 8 blocks), long rows, ties everywhere, duplicates,
+negative cosine distances; and the form that spreads a merge over the whole GPU."""
 
 import numpy as np
 import pytest
 
 import cuhc_b200 as C
 from _data import blobs, grid, normal
+from cuhc_b200 import _lib
+from cuhc_b200._linkage import _dense_with_options
 
 pytestmark = pytest.mark.gpu
 
@@ -76,6 +79,34 @@ def test_merges_bit_for_bit(name, method, metric):
     dist = C.pairwise_distances(X, metric=metric)
     got = C.linkage(X, method, metric=metric, algorithm="dense")
     np.testing.assert_array_equal(got, merge_all(dist, method))
+
+
+@pytest.mark.parametrize("method, metric", [("single", "euclidean"), ("complete", "manhattan"),
+                                            ("average", "cosine"), ("ward", "euclidean")])
+@pytest.mark.parametrize("name", CASES)
+def test_wide_merges_bit_for_bit(name, method, metric):
+    """The form for many slots, at every size."""
+    X = CASES[name]()
+    dist = C.pairwise_distances(X, metric=metric)
+    got = _dense_with_options(X, method, metric, resident_slots=0)
+    np.testing.assert_array_equal(got, merge_all(dist, method))
+
+
+@pytest.mark.parametrize("n, d", [(7168, 2), (7169, 2), (3072, 65), (3073, 65)])
+def test_forms_agree_around_their_line(n, d):
+    X = np.round(normal(n, d, seed=n) * 300).astype(np.float32)  # ties among long rows
+    got = C.linkage(X, "complete")
+    for slots in (0, n):
+        np.testing.assert_array_equal(_dense_with_options(X, "complete", resident_slots=slots), got)
+
+
+@pytest.mark.parametrize("slots", [0, 300])
+def test_non_finite_distances_end_either_form(slots):
+    X = normal(300, 4, seed=10)
+    X[7] = 3e38  # its squared differences overflow: no finite distance
+    tree = np.empty((299, 4))
+    assert _lib.lib.cuhc_linkage_dense_with_options(
+        _lib.float_ptr(X), 300, 4, 0, 2.0, 1, slots, _lib.double_ptr(tree)) < 0
 
 
 def test_long_rows():
