@@ -61,6 +61,9 @@ lib.cuhc_screen_counters.restype = _int
 lib.cuhc_screen_counters.argtypes = [ctypes.POINTER(ctypes.c_uint64), _int]
 lib.cuhc_set_screen.restype = _int
 lib.cuhc_set_screen.argtypes = [_int]
+lib.cuhc_ward_rnn_with_lists.restype = _int
+lib.cuhc_ward_rnn_with_lists.argtypes = [_f32, _int, _int, _float, _int, _f64,
+                                         ctypes.POINTER(_int)]
 lib.cuhc_linkage_dense_with_options.restype = _int
 lib.cuhc_linkage_dense_with_options.argtypes = [_f32, _int, _int, _int, _float, _int, _int, _f64]
 lib.cuhc_set_optional_memory.restype = _int

@@ -6,6 +6,8 @@ Mirrors the reference's python/cuhc/_linkage.py: the same id tables
 fcluster / cut_tree semantics (:152-216).
 """
 
+import ctypes
+
 import numpy as np
 
 from . import _lib
@@ -91,6 +93,19 @@ def _ward_rnn_with_options(X, min_progress, dense_below=0, allow_dense=True):
         _lib.float_ptr(X), n, X.shape[1], float(min_progress), int(dense_below),
         int(bool(allow_dense)), _lib.double_ptr(tree)))
     return tree
+
+
+def _ward_rnn_with_lists(X, lists_above, min_progress=0.0):
+    """Test hook: (tree, rounds that searched only some of the clusters) of Ward by
+    RNN rounds with nearest neighbours kept above a cluster count."""
+    X = as_points(X, "X")
+    n = X.shape[0]
+    tree = np.empty((max(n - 1, 0), 4), dtype=np.float64)
+    rounds = ctypes.c_int()
+    _lib.check(_lib.lib.cuhc_ward_rnn_with_lists(
+        _lib.float_ptr(X), n, X.shape[1], float(min_progress), int(lists_above),
+        _lib.double_ptr(tree), ctypes.byref(rounds)))
+    return tree, rounds.value
 
 
 def _dense_with_options(X, method, metric="euclidean", p=2.0, resident_slots=-1):

@@ -499,6 +499,30 @@ int cuhc_ward_rnn_with_options(const float *hostPoints, int n, int d, float minP
   return st.code;
 }
 
+int cuhc_ward_rnn_with_lists(const float *hostPoints, int n, int d, float minProgress,
+                             int listsAbove, double *hostTree, int *listedRounds) {
+  if (n <= 0 || d <= 0 || !listedRounds)
+    return kErrorInvalidShape;
+  *listedRounds = 0;
+  if (n == 1)
+    return 0;
+  CallContext ctx;
+  StatusChain st;
+  st(ctx.status);
+  DeviceBuffer<float> points;
+  CUHC_TRY(st, points.allocate((size_t)n * d, ctx.stream));
+  CUHC_TRY(st, cudaMemcpyAsync(points.get(), hostPoints, points.bytes(), cudaMemcpyHostToDevice,
+                               ctx.stream));
+  RnnOptions options;
+  options.minProgress = minProgress;
+  options.listsAbove = listsAbove;
+  options.listedRounds = listedRounds;
+  PassStats stats;
+  CUHC_TRY(st, rnnWard(points.get(), n, d, options, hostTree, &stats, ctx.stream));
+  addStats(stats);
+  return st.code;
+}
+
 int cuhc_linkage_dense_with_options(const float *hostPoints, int n, int d, int metricId, float p,
                                     int linkageId, int residentSlots, double *hostTree) {
   const int invalid = validateLinkage(n, d, metricId, linkageId, kDense);

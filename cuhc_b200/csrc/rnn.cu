@@ -520,9 +520,11 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
   const bool screened =
       st.ok() && useScreen<SqEuclideanMetric>(d, kListK) && index.extentsWithin(kScreenMaxExtent);
   // Lists, where there is room for them.
-  bool canList = screened ? n > kSearchAllBelow
-                          : n >= kPlainListsFrom &&
-                                listPassFits<SqEuclideanMetric, WardWeight>(d, kListK);
+  const int listsAbove = options.listsAbove >= 0               ? options.listsAbove
+                         : screened || n >= kPlainListsFrom ? kSearchAllBelow
+                                                              : n;
+  bool canList =
+      n > listsAbove && (screened || listPassFits<SqEuclideanMetric, WardWeight>(d, kListK));
   for (int b = 0; b < 2; ++b)
     canList = canList && allocateOptional(st, listRep[b], (size_t)n * kListK, s) &&
               allocateOptional(st, listWeight[b], (size_t)n * kListK, s) &&
@@ -541,7 +543,7 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
     parts.release();
   }
   std::vector<int> roundEnd;
-  int m = n, merged = 0, cur = 0, rounds = 0;
+  int m = n, merged = 0, cur = 0, rounds = 0, listedRounds = 0;
   enum { kNone, kDense, kChain } tail = kNone;
   unsigned long long tilesSoFar = 0;
   while (st.ok() && m > 1) {
@@ -578,8 +580,9 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
     p.screenAudit = screenAuditWords();
     WardWeight w;
     w.value = sizeF[cur].get();
-    const bool listed = canList && m > kSearchAllBelow;
+    const bool listed = canList && m > listsAbove;
     if (rounds > 0 && listed) {
+      ++listedRounds;
       bool ordered = false;
       CUHC_TRY(st, index.selectRows(searchFlag.get(), nullptr, sizeF[cur].get(), &ordered));
       p.rowPos = index.rowPos.get();
@@ -665,6 +668,8 @@ int rnnWard(const float *devPoints, int n, int d, const RnnOptions &options, dou
       break;
     }
   }
+  if (options.listedRounds)
+    *options.listedRounds = listedRounds;
   int err = 0;
   CUHC_TRY(st, cudaMemcpyAsync(&err, error.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
   unsigned long long tileCount = 0;

@@ -7,11 +7,16 @@
 namespace cuhc {
 
 // Hand-over settings of the RNN rounds; the reference's RnnOptions
-// (rnn_ward.cuh:66-86) with the same defaults.
+// (rnn_ward.cuh:66-86) with the same defaults. listsAbove: the cluster count above
+// which nearest neighbours are kept across rounds (-1: rnn.cu's own lines).
+// listedRounds, if not null, receives the rounds that searched only the rows
+// whose list did not settle them.
 struct RnnOptions {
   float minProgress = 0.01f;
   int denseBelow = 0;
   bool allowDense = true;
+  int listsAbove = -1;
+  int *listedRounds = nullptr;
 };
 
 // Ward merge tree by rounds of reciprocal nearest neighbours on device points

@@ -169,6 +169,12 @@ int cuhc_mlp_train(const float *x, const float *y, int count, int epochs, int ba
  * change; returns CUHC_ERROR_INVALID_ALGORITHM for other values. */
 int cuhc_set_screen(int mode);
 
+/* Test hook: Ward by RNN rounds with the number of clusters above which nearest
+ * neighbours are kept across rounds (-1: the defaults). The tree is the same.
+ * *listedRounds receives the rounds that searched only some of the clusters. */
+int cuhc_ward_rnn_with_lists(const float *points, int numPoints, int numFeatures,
+                             float minProgress, int listsAbove, double *tree, int *listedRounds);
+
 /* Test hook: cuhc_linkage's dense algorithm with the number of points up to which
  * one resident thread-block cluster makes the merges (-1: the default); above it
  * every merge uses the whole GPU. The tree is the same. A cluster that does not

@@ -16,7 +16,7 @@ import pytest
 
 from _data import blobs, grid, normal
 from cuhc_b200 import _lib
-from cuhc_b200._linkage import _ward_rnn_with_options
+from cuhc_b200._linkage import _ward_rnn_with_lists, _ward_rnn_with_options
 
 pytestmark = pytest.mark.gpu
 f4, f8 = np.float32, np.float64
@@ -109,3 +109,54 @@ def test_rounds_match_full_searches(name, screen):
     keys = sorted(expected)
     np.testing.assert_allclose([got[k] for k in keys], [expected[k] for k in keys],
                                rtol=4 * 2.0 ** -23, atol=0)
+
+
+@pytest.mark.parametrize("screen", ["on", "off"])
+@pytest.mark.parametrize("name", CASES)
+def test_kept_lists_match_full_searches(name, screen):
+    """The same with lists kept down to the last clusters, as the default keeps them
+    above a few thousand."""
+    X = np.ascontiguousarray(CASES[name]())
+    expected = clusters(ward_rounds(X), len(X))
+    _lib.set_screen(screen)
+    try:
+        tree, rounds = _ward_rnn_with_lists(X, lists_above=1)
+        full, none = _ward_rnn_with_lists(X, lists_above=len(X))
+    finally:
+        _lib.set_screen("auto")
+    assert none == 0 and rounds >= (4 if len(X) > 100 else 1)
+    np.testing.assert_array_equal(tree, full)
+    got = tree_clusters(tree)
+    assert got.keys() == expected.keys()
+    keys = sorted(expected)
+    np.testing.assert_allclose([got[k] for k in keys], [expected[k] for k in keys],
+                               rtol=4 * 2.0 ** -23, atol=0)
+
+
+HARD = {
+    "heavy tails": lambda r: r.standard_t(1.5, (5000, 6)),
+    "nested scales": lambda r: np.cumsum(r.standard_normal((12, 400, 9))
+                                         * 0.1 ** np.arange(12)[:, None, None], 0).reshape(-1, 9),
+    "nearly equal gaps": lambda r: np.arange(4000.0)[:, None] + r.uniform(-1e-4, 1e-4, (4000, 1)),
+    "coarse far from the origin": lambda r: r.standard_normal((4000, 3)) + 4e4,
+    "quantised": lambda r: r.integers(0, 5, (4500, 5)),
+    "two chunks": lambda r: r.standard_normal((4000, 50)),
+    "tiny values": lambda r: r.standard_normal((3000, 4)) * 1e-15,
+    "huge values": lambda r: r.standard_normal((3000, 4)) * 1e16,
+}
+
+
+@pytest.mark.parametrize("screen", ["on", "off"])
+@pytest.mark.parametrize("name", HARD)
+def test_kept_lists_equal_full_searches(name, screen):
+    """Larger sets, whose rounds have many clusters: bit for bit against the rounds
+    that search every cluster (which the oracle above checks)."""
+    X = np.ascontiguousarray(HARD[name](np.random.default_rng(5)), dtype=f4)
+    _lib.set_screen(screen)
+    try:
+        tree, rounds = _ward_rnn_with_lists(X, lists_above=1)
+        full, none = _ward_rnn_with_lists(X, lists_above=len(X))
+    finally:
+        _lib.set_screen("auto")
+    assert none == 0 and rounds >= 4
+    np.testing.assert_array_equal(tree, full)

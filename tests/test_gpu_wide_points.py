@@ -7,6 +7,7 @@ import pytest
 
 import cuhc_b200 as C
 from _data import assert_same_dendrogram, blobs
+from cuhc_b200._linkage import _ward_rnn_with_lists
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -30,5 +31,8 @@ def test_batch():
 
 
 def test_ward():
-    X = blobs(2100, WIDE, centers=40, seed=2)  # enough clusters for lists
+    X = blobs(2100, WIDE, centers=40, seed=2)
     assert_same_dendrogram(C.linkage(X, "ward"), C.linkage(X, "ward", algorithm="dense"))
+    tree, listed = _ward_rnn_with_lists(X, lists_above=500)
+    assert listed == 0  # asked for, but there is no room
+    np.testing.assert_array_equal(tree, C.linkage(X, "ward"))
