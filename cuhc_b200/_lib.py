@@ -186,7 +186,8 @@ def set_screen_audit(on):
 
 def screen_audit():
     """Audit results since the last call (resets): pairs audited,
-    violations of the screen's guarantee D' <= s (must be 0), the smallest
+    violations of the screen's guarantee D' <= s (must be 0; in Ward's rounds
+    also pairs that a row needed but the screen left out), the smallest
     slack (s - D') / (e (|x|^2 + |y|^2)) (>= 0 required; about 0.5 or more
     means the modelled error bound holds with room), the largest gap of the
     screened bound below the FP64 value (relative to the norms, and

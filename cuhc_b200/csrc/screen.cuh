@@ -296,6 +296,15 @@ __device__ __forceinline__ float tf32Up(float x) {
   return __uint_as_float((__float_as_uint(x) + 0x1fffu) & ~0x1fffu);
 }
 
+// A Ward column's extra slot, 1 / (2 s_j) rounded up. Slots past the clusters
+// hold anything: size 1 does for them.
+__device__ __forceinline__ float columnExtra(float size) {
+  return tf32Up(size >= 1.0f ? 0.5f / size : 0.5f);
+}
+
+// A Ward row's extra slot for cap c: c rounded up with 2^-8 to spare.
+__device__ __forceinline__ float rowExtraFor(float cap) { return tf32Up(cap * (1.0f + 0x1p-8f)); }
+
 // Row operand of row tile point i: [-2 x (KC), N hi, N lo, 1, 1, indicators]
 // (the factor -2, exact, sits on the side built once per row tile). A nonzero
 // `extra` takes the first indicator slot.
@@ -421,12 +430,21 @@ __device__ __forceinline__ void buildColumnOperandCosine(const float *raw, const
 // the pair count, violations (D' > s + 2^-70) and the extrema described at
 // ScreenAuditWord into `words`. Off the timed path: nothing here runs unless
 // the audit is on, and it changes no result.
-template <class Metric, int KC, bool kKnn>
+//
+// Ward: a pair that weighs at most the row's threshold rowThr but is not a
+// candidate (the accumulator exceeds Fs) is a violation, whatever the accumulator
+// holds. In a row with a cap it holds D' less rowExtra / (2 s_j): the product of
+// the two extra slots is added back before D' <= s is tested and the figures are
+// taken, in pairs where that product is not so large that its own rounding in the
+// accumulator (2^-20 of it at most) exceeds the margin.
+template <class Metric, class Weight, int KC, bool kKnn>
 __device__ __noinline__ void auditTile(unsigned long long *words, uint32_t taddr, const Metric &m,
                                        const float *sA, const float *raw, const float *centre,
                                        int myRow, bool rowValid, int myComp, int firstCol, int n,
                                        const int *cOrig, const int *cComp, bool useComp,
-                                       float margin) {
+                                       float margin, const Weight &w, float rowVal, float rowThr,
+                                       float rowExtra, float Fs, const float *cVal) {
+  constexpr bool kSized = std::is_same<Weight, WardWeight>::value;
   unsigned long long pairs = 0, violations = 0;
   float minSlack = INFINITY, maxGap = -INFINITY, maxAbs = -INFINITY, exactAbs = -INFINITY,
         exactRel = -INFINITY;
@@ -481,8 +499,17 @@ __device__ __noinline__ void auditTile(unsigned long long *words, uint32_t taddr
         s = (double)acc;
         norms = ni + nj;
       }
-      const double dp = (double)v[c];
+      double dp = (double)v[c];
       ++pairs;
+      if (kSized) {
+        const float size = cVal[jj];
+        if (w.weight((float)s, rowVal, size) <= rowThr && v[c] > Fs)
+          ++violations;
+        const double product = (double)rowExtra * (double)columnExtra(size);
+        if (product * 0x1p-20 > (double)margin * norms)
+          continue;
+        dp += product;
+      }
       if (dp > s + 0x1p-70)
         ++violations;
       // The relative margin is the guarantee where it exceeds the absolute
@@ -668,13 +695,14 @@ __global__ void __launch_bounds__(kThreads, 2)
   const float myCap = kSized && kKnn && mySearch && p.radius ? p.radius[myPos] : INFINITY;
   const bool sizedPass = kSized && kKnn && p.radius != nullptr;
   bool sized = kSized && myCap < 1e30f;
+  float myExtra = sized ? rowExtraFor(myCap) : 0.0f;
   float myNorm = 0.0f; // k-NN: the row's centred squared norm
   if (consumer) {
     if constexpr (kCos)
       buildRowOperandCosine<KC>(sA, myRow, mySearch, myComp, ss, opA);
     else
       buildRowOperand<KC>(sA, centre, scale, myRow, mySearch, myComp, ss, opA,
-                          sized ? -tf32Up(myCap * (1.0f + 0x1p-8f)) : 0.0f);
+                          -myExtra);
     if (kKnn) {
       float nrm = 0.0f;
 #pragma unroll
@@ -873,9 +901,9 @@ __global__ void __launch_bounds__(kThreads, 2)
       // The row's threshold takes the cap's place in the product (a looser cap
       // would let every heavy-partner column through). No MMA is in flight.
       if (consumer && mySearch && rowThr < 1e30f) {
+        myExtra = rowExtraFor(rowThr);
         *reinterpret_cast<float *>(reinterpret_cast<char *>(opA) + (myRow >> 3) * kSbo +
-                                   (myRow & 7) * 16 + (KC + 4) / 4 * 128) =
-            -tf32Up(rowThr * (1.0f + 0x1p-8f));
+                                   (myRow & 7) * 16 + (KC + 4) / 4 * 128) = -myExtra;
         sized = true;
       }
       fenceProxyAsync();
@@ -1025,10 +1053,8 @@ __global__ void __launch_bounds__(kThreads, 2)
             if constexpr (kCos)
               buildColumnOperandCosine<KC>(raw, comp, cosC, q, oneHot, ss, b);
             else if constexpr (kSized) {
-              // Slots past the clusters hold anything: size 1 does for them.
               const float size = reinterpret_cast<const float *>(comp + kTile)[q];
-              buildColumnOperand<KC>(raw, comp, cen, scale, q, oneHot, ss, b,
-                                     tf32Up(size >= 1.0f ? 0.5f / size : 0.5f));
+              buildColumnOperand<KC>(raw, comp, cen, scale, q, oneHot, ss, b, columnExtra(size));
             } else
               buildColumnOperand<KC>(raw, comp, cen, scale, q, oneHot, ss, b);
         }
@@ -1145,8 +1171,10 @@ __global__ void __launch_bounds__(kThreads, 2)
             cand[2 * half + 1] = cb;
           }
           if (kAudit)
-            auditTile<Metric, KC, kKnn>(p.screenAudit, taddr, m, sA, raw, centre, myRow, myValid,
-                                        myComp, J * kTile, p.n, cOrig, cComp, useComp, margin);
+            auditTile<Metric, Weight, KC, kKnn>(
+                p.screenAudit, taddr, m, sA, raw, centre, myRow, myValid, myComp, J * kTile, p.n,
+                cOrig, cComp, useComp, margin, w, myVal, F > -INFINITY ? rowThr : -1.0f,
+                sized ? myExtra : 0.0f, Fs, cVal);
           // Done with accumulator s: the MMA of ordinal t + 2 may overwrite it
           // while this warp rechecks.
           tcgenFenceBefore();

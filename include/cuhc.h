@@ -216,7 +216,8 @@ int cuhc_set_screen_audit(int on);
 
 /* Audit results of the current device since the last call, decoded into the
  * first `count` of: pairs audited; pairs whose screened value D' exceeded
- * s + 2^-70 (the screen's guarantee; must be 0); the smallest slack
+ * s + 2^-70 (the screen's guarantee; must be 0), and in Ward's rounds pairs that
+ * a row's threshold needed but the screen left out; the smallest slack
  * (s - D') / (e (|x|^2 + |y|^2)) with x, y the centred coordinates and e the
  * screen's margin; the largest (s64 - D') / (|x|^2 + |y|^2); the largest
  * s64 - D'; the largest |s - s64| and |s - s64| / s64. NaN where nothing was

@@ -21,6 +21,7 @@ import cuhc_b200 as C
 from _data import blobs
 from cuhc_b200 import _lib
 from cuhc_b200._hdbscan import hdbscan_tree
+from cuhc_b200._linkage import _ward_rnn_with_lists
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -136,6 +137,24 @@ def test_ward_rounds(audited):
     _lib.set_screen("off")
     np.testing.assert_array_equal(C.linkage(X, "ward"), screened)
     assert audit["pairs"] > 0
+
+
+@pytest.mark.parametrize("data", ["blobs", "uneven", "heavy tails"])
+def test_ward_rounds_with_sizes(audited, data):
+    """Rounds whose rows hold a cap in the product: no pair that a row's threshold
+    needs is dropped, and the figures are those of D' itself (with the cap's share
+    left in it, the gap below the FP64 value is many times the norms)."""
+    rng = np.random.default_rng(9)
+    X = {"blobs": lambda: blobs(4000, 16, centers=8, seed=53),
+         "uneven": lambda: np.vstack([rng.standard_normal((3400, 6)) * 0.01,
+                                      rng.standard_normal((600, 6)) * 20]),
+         "heavy tails": lambda: rng.standard_t(2, (4000, 12))}[data]().astype(np.float32)
+    tree, rounds = _ward_rnn_with_lists(X, lists_above=8)
+    assert rounds > 3
+    audit = assert_bound_held(min_pairs=100_000)
+    assert audit["max_bound_gap_rel_norms"] < 0.05, audit
+    _lib.set_screen("off")
+    np.testing.assert_array_equal(_ward_rnn_with_lists(X, lists_above=len(X))[0], tree)
 
 
 def test_audit_reports_fp64_errors(audited):
