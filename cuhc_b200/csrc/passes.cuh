@@ -68,6 +68,16 @@ struct ColumnMeta {
   float *value;
 };
 
+// Position of row r of row tile I in a list pass, -1 when there is none. Only
+// Ward's list passes (kWeighted) search some of the rows.
+template <bool kWeighted>
+__device__ __forceinline__ int listRowPosition(const PassParams &p, int I, int r) {
+  if (kWeighted)
+    return p.rowPosition(I, r);
+  const int pos = I * kTile + r;
+  return pos < p.n ? pos : -1;
+}
+
 // Whether a k-NN row is done: its list holds k points at distance 0 and another
 // one is known to tie them, so nothing can change its values or its tie flag.
 // (Identical points, 20,000 x 2: every row went on through all column tiles,
@@ -85,7 +95,9 @@ __device__ __forceinline__ void refreshThresholds(const PassParams &p, const Met
   const int tid = threadIdx.x;
   float t = -INFINITY;
   if (tid < kTile) {
-    const int pos = p.rowPosition(rowTile, tid);
+    const int pos = kKnn ? listRowPosition<!std::is_same<Weight, PlainWeight>::value>(
+                               p, rowTile, tid)
+                         : p.rowPosition(rowTile, tid);
     // Padding slots and inactive rows never search.
     const bool valid = pos >= 0 && p.order[pos] >= 0 && (kKnn || !p.active || p.active[pos]);
     float thr, filter = -INFINITY;
@@ -311,7 +323,7 @@ __device__ __forceinline__ void knnEpilogue(const PassParams &p, const Metric &m
 #pragma unroll
   for (int r = 0; r < 8; ++r) {
     const int rowInTile = g.row(r);
-    const int rowPos = p.rowPosition(rowTile, rowInTile);
+    const int rowPos = listRowPosition<kWeighted>(p, rowTile, rowInTile);
     float *list = lists + rowInTile * k;
     const float F = sh.rowFilter[rowInTile];
     float mn = INFINITY;
@@ -327,12 +339,14 @@ __device__ __forceinline__ void knnEpilogue(const PassParams &p, const Metric &m
         return w.weight(m.finalize(a), rowVal[r], cm.value[g.col(c)]);
       return firstCol + g.col(c) == rowPos ? 0.0f : listValue(m.finalize(a));
     };
-    // The offers below run one lane at a time, so only pairs that can change
-    // the list get there: a lighter value than the k-th, or an equal one whose
-    // index may precede (kWeighted) or whose tie is not on record yet. Testing
-    // the filter alone (nothing for cosine, a bound for size 1 for Ward) took,
-    // whole calls of 20,000 x 48: single linkage cosine 109 ms, now 58; Ward of
-    // normal points 97, now 49; single linkage of identical points 55, now 12.5.
+    // The offers below run one lane at a time, so where the filter excludes too
+    // little (nothing for cosine, a bound for size 1 for Ward) only pairs that can
+    // change the list get there: a lighter value than the k-th, or an equal one
+    // whose index may precede (kWeighted) or whose tie is not on record yet. Whole
+    // calls of 20,000 x 48, by the filter alone and so: single linkage cosine 109 /
+    // 58 ms, Ward of normal points 97 / 49. With a close filter the values cost more
+    // than they save (HDBSCAN euclidean 60,000 x 48, 25 samples: list pass 27 / 32).
+    constexpr bool kByValue = kWeighted || !Metric::kHasFilter;
     unsigned pending = 0;
     if (rowPos >= 0) {
       const float kth = list[k - 1];
@@ -341,9 +355,12 @@ __device__ __forceinline__ void knnEpilogue(const PassParams &p, const Metric &m
       for (int c = 0; c < 8; ++c)
         if (firstCol + g.col(c) < n && colOrig[g.col(c)] >= 0 && m.filter(acc[r][c]) <= F &&
             !(kWeighted && firstCol + g.col(c) == rowPos)) {
-          const float v = offered(acc[r][c], c);
-          if (v < kth || (equals && v == kth))
-            pending |= 1u << c;
+          if (kByValue) {
+            const float v = offered(acc[r][c], c);
+            if (!(v < kth || (equals && v == kth)))
+              continue;
+          }
+          pending |= 1u << c;
         }
     }
     while (true) {

@@ -1223,7 +1223,10 @@ __global__ void __launch_bounds__(kThreads, 2)
                   }
                 }
               } else if (kKnn) {
-                const float value = J * kTile + jj == myPos ? 0.0f : listValue(m.finalize(acc));
+                // (A squared distance is never below +0, nor is its root.)
+                float value = J * kTile + jj == myPos ? 0.0f : m.finalize(acc);
+                if (kCos)
+                  value = listValue(value);
                 // Offer to the row's list (the k-th value kept in a register):
                 // a value below the k-th enters, and the boundary-tie flag
                 // follows knnOffer (passes.cuh): an insertion evicts the old
