@@ -114,8 +114,9 @@ def load_radius_model(path=MODEL_PATH):
 
 
 def radius_stats():
-    """Since the last call: rows given a radius ('proposed'), rows settled by
-    the capped pass ('certified'), tiles computed by the capped passes
+    """Since the last call: rows of searching components ('proposed', whether or
+    not the kept lists spare their own search), those whose edge the radius proves
+    ('certified'), tiles computed by the capped passes
     ('capped_tiles') and by the fallback passes ('fallback_tiles')."""
     out = (ctypes.c_uint64 * 4)()
     _lib.check(_L.cuhc_radius_stats(out, 4))

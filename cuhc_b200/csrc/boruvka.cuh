@@ -238,7 +238,7 @@ static __global__ void chooseRows(const float *__restrict__ bound,
 }
 
 // Learned radius: rows of components that sit the round out are not proposed
-// (radius -1); counts the others.
+// (radius -1); counts the others, rows that need no search themselves included.
 static __global__ void proposeRows(const int *__restrict__ order, const int *__restrict__ comp,
                                    Participation who, int n, float *__restrict__ radius,
                                    unsigned long long *__restrict__ proposed) {

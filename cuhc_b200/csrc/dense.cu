@@ -189,7 +189,8 @@ __device__ __forceinline__ unsigned long long scanRow(const float *__restrict__ 
 __global__ void __launch_bounds__(kMergeThreads)
     denseMerges(float *__restrict__ dist, int n, int perBlock, int linkage,
                 const float *__restrict__ nearDist0, const int *__restrict__ nearSlot0,
-                const int *__restrict__ initialSize, MergeRecord *__restrict__ merges, int *__restrict__ mergeCount) {
+                const int *__restrict__ initialSize, MergeRecord *__restrict__ merges,
+                int *__restrict__ mergeCount) {
   extern __shared__ __align__(16) unsigned char dense_shared[];
   __shared__ MergeNote notes[2][kClusterBlocks];
   __shared__ unsigned long long warpBest[kMergeThreads / 32], warpRow[kMergeThreads / 32];

@@ -258,7 +258,8 @@ __global__ void updateLists(WardLists in, WardLists out, const int *__restrict__
                             const int *__restrict__ slotOfRep, const float *__restrict__ cent,
                             const float *__restrict__ size, const int *__restrict__ nextRep,
                             const unsigned char *__restrict__ changed, int d, WardRounding r,
-                            unsigned long long *nearest, unsigned char *__restrict__ flag, float *__restrict__ cap) {
+                            unsigned long long *nearest, unsigned char *__restrict__ flag,
+                            float *__restrict__ cap) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m)
     return;

@@ -144,7 +144,11 @@ int cuhc_trees_batched_device(const float *devicePoints, const long long *offset
  * exp(prediction + offset)); params NULL switches the proposal off. */
 int cuhc_set_radius_model(const float *params, float offset);
 /* Since the last call (first `count` of: rows proposed, rows certified,
- * tiles of the capped passes, tiles of the fallback passes). */
+ * tiles of the capped passes, tiles of the fallback passes). A row counts as
+ * proposed once per round in which its component searches, also when what it
+ * knows from the kept lists spares its own search; rows of components that sit
+ * a round out do not count. Certified rows are those of them whose lightest known
+ * or found edge the radius proves. */
 int cuhc_radius_stats(unsigned long long *out, int count);
 /* The pipeline shape (ring slots, copy lead) that the shape tuner chose for
  * the latest screened k-NN pass (0, 0 before any). No counterpart in the
