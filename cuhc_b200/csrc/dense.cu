@@ -47,10 +47,11 @@ constexpr int kClusterBlocks = 8, kMergeThreads = 512, kMinSlots = 128;
 // many others' nearest, the more so the more features there are. Average linkage
 // of normal points in ms, cluster / whole GPU: 2 features 4,000 points 23 / 46,
 // 8,000 70 / 121, 20,000 337 / 507; 64 features 4,000 35 / 48, 6,000 73 / 83, 8,000
-// 121 / 125, 20,000 698 / 526; 300 features 4,000 47 / 49, 5,000 72 / 65, 20,000
-// 1,443 / 538; 1,000 features 3,072 34 / 37, 4,096 55 / 49. Ward of 400-fold
-// duplicates, 8 features: 6,000 75 / 85, 8,000 118 / 115.
-inline int residentSlotsFor(int d) { return d <= 64 ? 7168 : 3072; }
+// 121 / 125, 20,000 698 / 526; 128 features 4,096 37 / 47, 6,144 81 / 82, 7,168
+// 113 / 103; 300 features 4,000 47 / 49, 5,000 72 / 65, 20,000 1,443 / 538; 1,000
+// features 3,072 34 / 37, 4,096 55 / 49. Ward of 400-fold duplicates, 8 features:
+// 6,000 75 / 85, 8,000 118 / 115.
+inline int residentSlotsFor(int d) { return d <= 64 ? 7168 : d <= 128 ? 5120 : 3072; }
 // The wide form: threads of the reducing block, merges per captured graph.
 constexpr int kReduceThreads = 1024, kStepsPerGraph = 64;
 enum LinkageKind : int { kSingleL = 0, kCompleteL = 1, kAverageL = 2, kWardL = 3 };

@@ -92,7 +92,8 @@ def test_wide_merges_bit_for_bit(name, method, metric):
     np.testing.assert_array_equal(got, merge_all(dist, method))
 
 
-@pytest.mark.parametrize("n, d", [(7168, 2), (7169, 2), (3072, 65), (3073, 65)])
+@pytest.mark.parametrize("n, d", [(7168, 2), (7169, 2), (5120, 65), (5121, 65), (3072, 129),
+                                  (3073, 129)])
 def test_forms_agree_around_their_line(n, d):
     X = np.round(normal(n, d, seed=n) * 300).astype(np.float32)  # ties among long rows
     got = C.linkage(X, "complete")
